@@ -3,6 +3,7 @@
 #include "../../include/fta.h"
 
 #include "fta_kernels.h"
+#include "native_api.h"
 #include "tmap.h"
 
 namespace {
@@ -77,51 +78,26 @@ int map_bias(CUtensorMap* m, const FtaProblem* p, const FtaTensor4* t, int box_k
 
 size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
-int num_sms() {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
+size_t plane_bytes(const FtaProblem* p) { return static_cast<size_t>(p->B) * p->H * p->L2 * p->L2 * sizeof(float); }
+size_t dq32_bytes(const FtaProblem* p) {
+  return static_cast<size_t>(p->B) * p->H * p->L1 * p->L2 * p->D * sizeof(float);
 }
-
-}  // namespace
-
-namespace fta {
-int record_cuda_error(int cuda_error) { return cuda_fail(cuda_error); }
-}  // namespace fta
-
-extern "C" {
-
-int fta_version(void) { return 200; }
-
-const char* fta_strerror(int code) {
-  switch (code) {
-    case FTA_OK: return "ok";
-    case FTA_ERR_NULL: return "a required pointer is NULL";
-    case FTA_ERR_SHAPE: return "bad shape: sizes must be positive and L2 a multiple of 8 (of 128 without fta_mask_bias)";
-    case FTA_ERR_HEAD_DIM: return "unsupported head dimension: D must be 32 or 64";
-    case FTA_ERR_DTYPE: return "unsupported dtype: fp16 or bf16 only";
-    case FTA_ERR_STRIDE: return "bad stride: D stride must be 1, other strides positive multiples of 8 elements";
-    case FTA_ERR_ALIGN: return "every device pointer must be 16-byte aligned";
-    case FTA_ERR_WORKSPACE: return "workspace too small or misaligned";
-    case FTA_ERR_TENSOR_MAP: return "the driver refused a TMA tensor map";
-    case FTA_ERR_CUDA: return "a CUDA runtime call failed";
-    case FTA_ERR_DEVICE: return "a bounded device-side wait ran out (status word non-zero)";
-    case FTA_ERR_TOO_LARGE: return "size beyond a documented maximum";
-    default: return "unknown error";
-  }
+// float32 dQ accumulator, dBias planes, key-major copy of the bias (16-bit, whole blocks)
+size_t workspace_bytes(const FtaProblem* p, int nplanes) {
+  const size_t l2p = static_cast<size_t>(padded_l2(p));
+  return align256(dq32_bytes(p)) + align256(plane_bytes(p) * nplanes) +
+         align256(static_cast<size_t>(p->B) * p->H * l2p * l2p * 2);
 }
+int plan_planes(const FtaProblem* p) { return fta::bwd_num_planes(p->B, p->H, p->L1, p->L2, p->D, fta::num_sms()); }
 
-int fta_last_cuda_error(void) { return g_last_cuda_error; }
-
-int fta_forward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
-                const FtaTensor4* bias, float sm_scale, const FtaTensor5* o, void* o_resid, float* lse,
-                int32_t* status, void* stream) {
+int forward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
+            const FtaTensor4* bias, float sm_scale, const FtaTensor5* o, void* o_resid, float* lse, fta::Status status,
+            cudaStream_t stream) {
   int rc = check_problem(prob);
   if (rc) return rc;
-  if ((rc = check_t5(q)) || (rc = check_t5(k)) || (rc = check_t5(v)) || (rc = check_t5(o)) ||
-      (rc = check_t4(bias)))
+  if ((rc = check_t5(q)) || (rc = check_t5(k)) || (rc = check_t5(v)) || (rc = check_t5(o)) || (rc = check_t4(bias)))
     return rc;
-  if (!lse || !status) return FTA_ERR_NULL;
+  if (!status.word) return FTA_ERR_NULL;
   if (!aligned16(lse) || !aligned16(o_resid)) return FTA_ERR_ALIGN;
   fta::FwdArgs a;
   if ((rc = map5(&a.tmQ, prob, q)) || (rc = map5(&a.tmK, prob, k)) || (rc = map5(&a.tmV, prob, v)) ||
@@ -139,12 +115,12 @@ int fta_forward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* k
   a.bf16 = prob->dtype == FTA_BF16;
   for (int i = 0; i < 4; ++i) a.so[i] = o->stride[i];
   a.sm_scale = sm_scale;
-  if (const int e = fta::launch_fwd(a, static_cast<cudaStream_t>(stream))) return cuda_fail(e);
+  if (const int e = fta::launch_fwd(a, stream)) return cuda_fail(e);
   return FTA_OK;
 }
 
-int fta_bwd_preprocess(const FtaProblem* prob, const FtaTensor5* o, const void* o_resid, const FtaTensor5* dout,
-                       float* delta, void* stream) {
+int preprocess(const FtaProblem* prob, const FtaTensor5* o, const void* o_resid, const FtaTensor5* dout, float* delta,
+               cudaStream_t stream) {
   int rc = check_problem(prob);
   if (rc) return rc;
   if ((rc = check_t5(o)) || (rc = check_t5(dout))) return rc;
@@ -158,69 +134,34 @@ int fta_bwd_preprocess(const FtaProblem* prob, const FtaTensor5* o, const void* 
   const int l2p = padded_l2(prob);
   if (l2p != prob->L2) {
     // the entries of queries past L2 (whole 128-blocks are read by the backward kernel) must be finite
-    const cudaError_t e = cudaMemsetAsync(delta, 0, sizeof(float) * static_cast<size_t>(prob->B) * prob->H * prob->L1 * l2p,
-                                          static_cast<cudaStream_t>(stream));
+    const cudaError_t e = cudaMemsetAsync(
+        delta, 0, sizeof(float) * static_cast<size_t>(prob->B) * prob->H * prob->L1 * l2p, stream);
     if (e != cudaSuccess) return cuda_fail(e);
   }
   if (const int e = fta::launch_preprocess(o->ptr, o_resid, so, dout->ptr, sd, delta, l2p, prob->B, prob->H, prob->L1,
-                                           prob->L2, prob->D, prob->dtype == FTA_BF16,
-                                           static_cast<cudaStream_t>(stream)))
+                                           prob->L2, prob->D, prob->dtype == FTA_BF16, stream))
     return cuda_fail(e);
   return FTA_OK;
 }
 
-int fta_mask_bias(const FtaProblem* prob, const FtaTensor4* bias, const uint8_t* key_mask, void* out, void* stream) {
-  int rc = check_problem(prob);
-  if (rc) return rc;
-  if ((rc = check_t4(bias))) return rc;
-  if (!out) return FTA_ERR_NULL;
-  if (!aligned16(out) || reinterpret_cast<uintptr_t>(key_mask) % 8 != 0) return FTA_ERR_ALIGN;
-  long long sb[4];
-  for (int i = 0; i < 4; ++i) sb[i] = bias->stride[i];
-  if (const int e = fta::launch_mask_bias(bias->ptr, sb, key_mask, out, prob->B, prob->H, prob->L2, padded_l2(prob),
-                                          prob->dtype == FTA_BF16, static_cast<cudaStream_t>(stream)))
-    return cuda_fail(e);
-  return FTA_OK;
-}
-
-int fta_bwd_num_planes(const FtaProblem* prob) {
-  if (check_problem(prob)) return 0;
-  return fta::bwd_num_planes(prob->B, prob->H, prob->L1, prob->L2, prob->D, num_sms());
-}
-
-size_t fta_bwd_workspace_bytes(const FtaProblem* prob) {
-  if (check_problem(prob)) return 0;
-  const size_t rows = static_cast<size_t>(prob->B) * prob->H * prob->L1 * prob->L2;
-  const size_t plane = static_cast<size_t>(prob->B) * prob->H * prob->L2 * prob->L2 * sizeof(float);
-  const size_t l2p = static_cast<size_t>(padded_l2(prob));
-  return align256(rows * prob->D * sizeof(float)) + align256(plane * fta_bwd_num_planes(prob)) +
-         align256(static_cast<size_t>(prob->B) * prob->H * l2p * l2p * 2);  // + key-major copy of the bias (16-bit, whole blocks)
-}
-
-int fta_backward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
-                 const FtaTensor4* bias, const FtaTensor5* dout, const float* lse, const float* delta,
-                 float sm_scale, const FtaTensor5* dq, const FtaTensor5* dk, const FtaTensor5* dv,
-                 float* dbias_f32, void* dbias_cast, void* workspace, size_t workspace_bytes, int32_t* status,
-                 void* stream) {
-  int rc = check_problem(prob);
-  if (rc) return rc;
+int backward(const FtaProblem* prob, int nplanes, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
+             const FtaTensor4* bias, const FtaTensor5* dout, const float* lse, const float* delta, float sm_scale,
+             const FtaTensor5* dq, const FtaTensor5* dk, const FtaTensor5* dv, float* dbias_f32, void* dbias_cast,
+             void* workspace, size_t have_bytes, fta::Status status, cudaStream_t st) {
+  int rc;
   if ((rc = check_t5(q)) || (rc = check_t5(k)) || (rc = check_t5(v)) || (rc = check_t5(dout)) ||
       (rc = check_t5(dq)) || (rc = check_t5(dk)) || (rc = check_t5(dv)) || (rc = check_t4(bias)))
     return rc;
-  if (!lse || !delta || !dbias_f32 || !status || !workspace) return FTA_ERR_NULL;
+  if (!lse || !delta || !dbias_f32 || !status.word || !workspace) return FTA_ERR_NULL;
   // the kernel fetches the statistics with 512-byte bulk copies and the epilogue writes dBias with
   // 16-byte stores
   if (!aligned16(lse) || !aligned16(delta) || !aligned16(dbias_f32) || !aligned16(dbias_cast)) return FTA_ERR_ALIGN;
-  if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0 || workspace_bytes < fta_bwd_workspace_bytes(prob))
+  if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0 || have_bytes < workspace_bytes(prob, nplanes))
     return FTA_ERR_WORKSPACE;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t rows = static_cast<size_t>(prob->B) * prob->H * prob->L1 * prob->L2;
-  const size_t dq_bytes = rows * prob->D * sizeof(float);
-  const long long plane_elems = static_cast<long long>(prob->B) * prob->H * prob->L2 * prob->L2;
   float* dq32 = static_cast<float*>(workspace);
-  float* planes = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(dq_bytes));
-  const int nplanes = fta_bwd_num_planes(prob);
-  void* bias_t = reinterpret_cast<uint8_t*>(planes) + align256(static_cast<size_t>(plane_elems) * 4 * nplanes);
+  float* planes = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(dq32_bytes(prob)));
+  void* bias_t = reinterpret_cast<uint8_t*>(planes) + align256(plane_bytes(prob) * nplanes);
   const bool bf16 = prob->dtype == FTA_BF16;
 
   fta::BwdArgs a;
@@ -254,7 +195,8 @@ int fta_backward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* 
   a.dq32 = dq32;
   a.dk = dk->ptr;
   a.dv = dv->ptr;
-  a.status = status;
+  a.status = status.word;
+  a.nplanes = nplanes;
   a.B = prob->B;
   a.H = prob->H;
   a.L1 = prob->L1;
@@ -278,9 +220,110 @@ int fta_backward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* 
   if (const int e = fta::launch_bwd(a, st)) return cuda_fail(e);
   if (g_prof_stop) cudaEventRecord(g_prof_stop, st);
   if (const int e = fta::launch_bwd_epilogue(dq32, dq->ptr, sdq, prob->B, prob->H, prob->L1, prob->L2, prob->D,
-                                             sm_scale, planes, nplanes, dbias_f32, dbias_cast, bf16, st))
+                                             sm_scale, planes, nplanes, dbias_f32, dbias_cast, bf16, status, st))
     return cuda_fail(e);
   return FTA_OK;
+}
+
+
+}  // namespace
+
+namespace fta {
+
+int record_cuda_error(int cuda_error) { return cuda_fail(cuda_error); }
+
+int native_forward(const FtaProblem& prob, const FtaTensor5& q, const FtaTensor5& k, const FtaTensor5& v,
+                   const FtaTensor4& bias, float sm_scale, const FtaTensor5& o, void* o_resid, float* lse,
+                   StatusPair status, cudaStream_t stream) {
+  return forward(&prob, &q, &k, &v, &bias, sm_scale, &o, o_resid, lse, {status.word, status.mirror}, stream);
+}
+
+int native_backward_plan(const FtaProblem& prob, BackwardPlan* plan) {
+  if (const int rc = check_problem(&prob)) return rc;
+  plan->nplanes = plan_planes(&prob);
+  plan->workspace_bytes = workspace_bytes(&prob, plan->nplanes);
+  plan->delta_bytes = sizeof(float) * static_cast<size_t>(prob.B) * prob.H * prob.L1 * padded_l2(&prob);
+  return FTA_OK;
+}
+
+int native_backward(const FtaProblem& prob, const BackwardPlan& plan, const FtaTensor5& q, const FtaTensor5& k,
+                    const FtaTensor5& v, const FtaTensor4& bias, const FtaTensor5& o, const void* o_resid,
+                    const FtaTensor5& dout, const float* lse, float sm_scale, const FtaTensor5& dq,
+                    const FtaTensor5& dk, const FtaTensor5& dv, float* dbias_f32, void* dbias_cast, void* workspace,
+                    StatusPair status, cudaStream_t stream) {
+  float* delta = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + plan.workspace_bytes);
+  if (const int rc = preprocess(&prob, &o, o_resid, &dout, delta, stream)) return rc;
+  return backward(&prob, plan.nplanes, &q, &k, &v, &bias, &dout, lse, delta, sm_scale, &dq, &dk, &dv, dbias_f32,
+                  dbias_cast, workspace, plan.workspace_bytes, {status.word, status.mirror}, stream);
+}
+
+}  // namespace fta
+
+extern "C" {
+
+int fta_version(void) { return 200; }
+
+const char* fta_strerror(int code) {
+  switch (code) {
+    case FTA_OK: return "ok";
+    case FTA_ERR_NULL: return "a required pointer is NULL";
+    case FTA_ERR_SHAPE: return "bad shape: sizes must be positive and L2 a multiple of 8 (of 128 without fta_mask_bias)";
+    case FTA_ERR_HEAD_DIM: return "unsupported head dimension: D must be 32 or 64";
+    case FTA_ERR_DTYPE: return "unsupported dtype: fp16 or bf16 only";
+    case FTA_ERR_STRIDE: return "bad stride: D stride must be 1, other strides positive multiples of 8 elements";
+    case FTA_ERR_ALIGN: return "every device pointer must be 16-byte aligned";
+    case FTA_ERR_WORKSPACE: return "workspace too small or misaligned";
+    case FTA_ERR_TENSOR_MAP: return "the driver refused a TMA tensor map";
+    case FTA_ERR_CUDA: return "a CUDA runtime call failed";
+    case FTA_ERR_DEVICE: return "a bounded device-side wait ran out (status word non-zero)";
+    case FTA_ERR_TOO_LARGE: return "size beyond a documented maximum";
+    default: return "unknown error";
+  }
+}
+
+int fta_last_cuda_error(void) { return g_last_cuda_error; }
+
+int fta_forward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
+                const FtaTensor4* bias, float sm_scale, const FtaTensor5* o, void* o_resid, float* lse,
+                int32_t* status, void* stream) {
+  if (const int rc = check_problem(prob)) return rc;
+  if (!lse) return FTA_ERR_NULL;
+  return forward(prob, q, k, v, bias, sm_scale, o, o_resid, lse, {status, nullptr}, static_cast<cudaStream_t>(stream));
+}
+
+int fta_bwd_preprocess(const FtaProblem* prob, const FtaTensor5* o, const void* o_resid, const FtaTensor5* dout,
+                       float* delta, void* stream) {
+  return preprocess(prob, o, o_resid, dout, delta, static_cast<cudaStream_t>(stream));
+}
+
+int fta_mask_bias(const FtaProblem* prob, const FtaTensor4* bias, const uint8_t* key_mask, void* out, void* stream) {
+  int rc = check_problem(prob);
+  if (rc) return rc;
+  if ((rc = check_t4(bias))) return rc;
+  if (!out) return FTA_ERR_NULL;
+  if (!aligned16(out) || reinterpret_cast<uintptr_t>(key_mask) % 8 != 0) return FTA_ERR_ALIGN;
+  long long sb[4];
+  for (int i = 0; i < 4; ++i) sb[i] = bias->stride[i];
+  if (const int e = fta::launch_mask_bias(bias->ptr, sb, key_mask, out, prob->B, prob->H, prob->L2, padded_l2(prob),
+                                          prob->dtype == FTA_BF16, static_cast<cudaStream_t>(stream)))
+    return cuda_fail(e);
+  return FTA_OK;
+}
+
+int fta_bwd_num_planes(const FtaProblem* prob) { return check_problem(prob) ? 0 : plan_planes(prob); }
+
+size_t fta_bwd_workspace_bytes(const FtaProblem* prob) {
+  return check_problem(prob) ? 0 : workspace_bytes(prob, plan_planes(prob));
+}
+
+int fta_backward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
+                 const FtaTensor4* bias, const FtaTensor5* dout, const float* lse, const float* delta,
+                 float sm_scale, const FtaTensor5* dq, const FtaTensor5* dk, const FtaTensor5* dv,
+                 float* dbias_f32, void* dbias_cast, void* workspace, size_t workspace_bytes, int32_t* status,
+                 void* stream) {
+  if (const int rc = check_problem(prob)) return rc;
+  return backward(prob, plan_planes(prob), q, k, v, bias, dout, lse, delta, sm_scale, dq, dk, dv, dbias_f32, dbias_cast,
+                  workspace, workspace_bytes, {status, nullptr}, static_cast<cudaStream_t>(stream));
 }
 
 int fta_dbias_cast(const float* src, void* dst, int64_t n, int32_t dtype, void* stream) {

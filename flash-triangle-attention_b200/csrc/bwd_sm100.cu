@@ -861,17 +861,17 @@ int bwd_rows_per_cta(int D) { return D == 32 ? BwdCfg<32>::G : BwdCfg<64>::G; }
 // Number of private dBias planes == number of row blocks per (b,h,key block). Chosen so that the
 // grid (B*H * L2/128 * NP CTAs, one per SM at a time) fills whole waves of the device with
 // chains of nearly equal length, with as few planes as that allows.
-int bwd_num_planes(int B, int H, int L1, int L2, int D, int num_sms) {
+int bwd_num_planes(int B, int H, int L1, int L2, int D, int sms) {
   const int G = bwd_rows_per_cta(D);
   const int ngroups = (L1 + G - 1) / G;
   const long long base = static_cast<long long>(B) * H * ((L2 + 127) / 128);
   const int np_max = ngroups < 64 ? ngroups : 64;
   auto efficiency = [&](int np) {
     const long long ctas = base * np;
-    const long long waves = (ctas + num_sms - 1) / num_sms;
+    const long long waves = (ctas + sms - 1) / sms;
     const int chain = (L1 + np - 1) / np;  // rows of the longest chain
-    // time ~ waves * chain ; work ~ base * L1 / num_sms
-    return (static_cast<double>(base) * L1 / num_sms) / (static_cast<double>(waves) * chain);
+    // time ~ waves * chain ; work ~ base * L1 / sms
+    return (static_cast<double>(base) * L1 / sms) / (static_cast<double>(waves) * chain);
   };
   // The planes are updated in place all through the kernel, so their footprint should stay inside
   // the L2 cache. While it does (half of the 126 MB), take the best schedule, and the fewest planes
@@ -896,10 +896,7 @@ int bwd_num_planes(int B, int H, int L1, int L2, int D, int num_sms) {
 }
 
 int launch_bwd(const BwdArgs& a, cudaStream_t stream) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int NP = bwd_num_planes(a.B, a.H, a.L1, a.L2, a.D, sms);
+  const int NP = a.nplanes;
   if (a.D == 32) return a.bf16 ? launch_bwd_t<32, true>(a, NP, stream) : launch_bwd_t<32, false>(a, NP, stream);
   return a.bf16 ? launch_bwd_t<64, true>(a, NP, stream) : launch_bwd_t<64, false>(a, NP, stream);
 }

@@ -35,12 +35,37 @@ inline cudaError_t ensure_dynamic_smem(PerDeviceOnce& once, Kernel kern, int byt
   return e;
 }
 
+// SM count of the current device, looked up once per device (the attribute call costs more than the
+// rest of a launch's host arithmetic).
+inline int num_sms() {
+  static std::atomic<int> cached[PerDeviceOnce::kMaxDevices] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  const bool tracked = dev >= 0 && dev < PerDeviceOnce::kMaxDevices;
+  if (tracked) {
+    if (const int n = cached[dev].load(std::memory_order_relaxed)) return n;
+  }
+  int sms = 148;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && tracked)
+    cached[dev].store(sms, std::memory_order_relaxed);
+  return sms;
+}
+
+// The status word of a launch and its optional mirror in mapped host memory. A failed wait leaves its code
+// in the word; the forward kernel (as it tears down) and the last kernel of a backward pass copy a word that
+// is not zero to the mirror themselves, so the host can look for a failure without a copy or a
+// synchronisation on the stream.
+struct Status {
+  int* word;
+  int* mirror;  // nullptr: no mirror
+};
+
 struct FwdArgs {
   CUtensorMap tmQ, tmK, tmV, tmBias;
   void* o;
   void* o_resid;  // nullptr, or the rounding residual of O with O's strides
-  float* lse;
-  int* status;
+  float* lse;     // nullptr: no statistics (no backward pass will follow)
+  Status status;
   int B, H, L1, L2, D;
   bool bf16;
   long long so[4];  // element strides of O (and of the residual) over (B, H, L1, L2)
@@ -60,13 +85,14 @@ struct BwdArgs {
   void* dv;
   int* status;
   int B, H, L1, L2, D;
+  int nplanes;  // bwd_num_planes()
   bool bf16;
   long long sdk[4], sdv[4];  // element strides of dK, dV over (B, H, L1, L2)
   float sm_scale;
 };
 int launch_bwd(const BwdArgs& a, cudaStream_t stream);
 int bwd_rows_per_cta(int D);
-int bwd_num_planes(int B, int H, int L1, int L2, int D, int num_sms);
+int bwd_num_planes(int B, int H, int L1, int L2, int D, int sms);
 
 // delta[(b,h,i), j] = sum_d (O[.,d] + R[.,d]) * dO[.,d]; `o_resid` (R, strides of O) may be nullptr;
 // `delta_pitch` = elements between rows (b,h,i) of delta (L2 rounded up to 128)
@@ -90,7 +116,7 @@ int launch_bwd_prologue(const void* bias, const long long sb[4], void* bias_t, i
 // dbias_f32[bh][query][key] = sum_p planes[p][bh][key][query] in plane order, optional rounded copy
 int launch_bwd_epilogue(const float* dq32, void* dq, const long long sdq[4], int B, int H, int L1, int L2, int D,
                         float scale, const float* planes, int nplanes, float* dbias_f32, void* dbias_cast, bool bf16,
-                        cudaStream_t stream);
+                        Status status, cudaStream_t stream);
 
 // out = sum over r of parts[r][0..n) (rank order), float32 and / or rounded to 16 bits; `parts`: device
 // array of `nranks` device pointers (peer mappings included); n a multiple of 8

@@ -69,8 +69,8 @@ struct FwdCfg {
 struct FwdParams {
   void* o;
   void* o_resid;  // optional: the part of O lost in rounding to 16 bits, same layout as O
-  float* lse;
-  int* status;
+  float* lse;     // nullptr: no statistics
+  Status status;
   int H, L1, L2;
   long long so_b, so_h, so_i, so_j;  // element strides of O (D stride is 1)
   float scale;                       // sm_scale
@@ -126,7 +126,7 @@ fta_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   // (kept a run-time value: as a compile-time constant it changes the code the compiler generates
   // for the softmax loop, measurably for the worse)
   auto unit_gp = [&](int u) { return unit_i0(u) < p.L1 ? G : 0; };
-  const WaitCtx w{smem_u32(abort_flag), p.status};
+  const WaitCtx w{smem_u32(abort_flag), p.status.word};
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -484,7 +484,7 @@ fta_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
               }
             }
           }
-          if (i < p.L1) {
+          if (i < p.L1 && p.lse != nullptr) {
             float m_safe_out = m_safe;
             // softmax statistics for the backward pass: -max (natural-log units) and -log2(sum).
             // Kept apart: their sum in one float would lose log2(sum) when |max| is huge.
@@ -511,6 +511,8 @@ fta_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag) __nanosleep(20000);  // let copies already in flight land before the CTA exits
+  if (threadIdx.x == 0 && (*abort_flag || (blockIdx.x | blockIdx.y | blockIdx.z) == 0))
+    publish_status(p.status.word, p.status.mirror);
   if (warp == 0) tmem_dealloc(tbase, 512);
 }
 
@@ -541,16 +543,11 @@ int launch_fwd_t(const FwdArgs& a, cudaStream_t stream) {
   // across row groups.
   const int ngroups = (a.L1 + C::G - 1) / C::G;
   const long long per = static_cast<long long>((a.L2 + 127) / 128) * a.B * a.H;
-  int sms = 148;
-  {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  }
+  const int sms = num_sms();
   int best_gy = 1;
   {
     double best = 0.0;
-    const int gy_max = ngroups;
+    const int gy_max = ngroups < 96 ? ngroups : 96;  // beyond that the last wave is a small part of any schedule
     // first pass: best efficiency; second: smallest gy close to it
     for (int pass = 0; pass < 2; ++pass) {
       for (int gy = 1; gy <= gy_max; ++gy) {

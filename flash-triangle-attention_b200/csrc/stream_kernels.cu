@@ -453,8 +453,9 @@ __global__ void __launch_bounds__(256) bwd_epilogue_kernel(const float* __restri
                                                            long long s_h, long long s_i, long long s_j, float scale,
                                                            int dq_blocks, const float* __restrict__ planes, int nplanes,
                                                            int BH, float* __restrict__ out_f32,
-                                                           uint16_t* __restrict__ out_cast) {
+                                                           uint16_t* __restrict__ out_cast, Status status) {
   __shared__ float tile[64][65];  // [key][query]
+  if (blockIdx.x == 0 && threadIdx.x == 0) publish_status(status.word, status.mirror);
   if (static_cast<int>(blockIdx.x) < dq_blocks) {
     constexpr int LPR = kD / 8;
     const long long nthreads = static_cast<long long>(dq_blocks) * blockDim.x;
@@ -561,13 +562,6 @@ __global__ void __launch_bounds__(256) bwd_epilogue_kernel(const float* __restri
   }
 }
 
-int num_sms() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 int grid_for(long long work_items, int threads) {
   long long blocks = (work_items + threads - 1) / threads;
   const long long cap = static_cast<long long>(num_sms()) * 8;  // a multiple of the SM count
@@ -643,7 +637,7 @@ int launch_bwd_prologue(const void* bias, const long long sb[4], void* bias_t, i
 
 int launch_bwd_epilogue(const float* dq32, void* dq, const long long sdq[4], int B, int H, int L1, int L2, int D,
                         float scale, const float* planes, int nplanes, float* dbias_f32, void* dbias_cast, bool bf16,
-                        cudaStream_t stream) {
+                        Status status, cudaStream_t stream) {
   const long long rows = static_cast<long long>(B) * H * L1 * L2;
   const int dq_blocks = grid_for(rows * (D / 8), 256);
   const int db_blocks = ((L2 + 63) / 64) * ((L2 + 63) / 64) * B * H;
@@ -653,7 +647,7 @@ int launch_bwd_epilogue(const float* dq32, void* dq, const long long sdq[4], int
   const bool dense = is_dense(sdq, H, L1, L2, D);
   auto go = [&](auto kern) {
     kern<<<grid, 256, 0, stream>>>(dq32, out, rows, H, L1, L2, sdq[0], sdq[1], sdq[2], sdq[3], scale, dq_blocks,
-                                   planes, nplanes, B * H, dbias_f32, cast);
+                                   planes, nplanes, B * H, dbias_f32, cast, status);
   };
   auto pick = [&](auto d_tag, auto bf_tag) {
     constexpr int DD = decltype(d_tag)::value;

@@ -159,6 +159,14 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, co
   return __all_sync(0xffffffffu, ok);
 }
 
+// Host-visible copy of a status word (see Status in fta_kernels.h): one thread, nothing to do while the
+// word is zero.
+__device__ __forceinline__ void publish_status(const int* word, int* mirror) {
+  if (mirror == nullptr) return;
+  const int code = *reinterpret_cast<const volatile int*>(word);
+  if (code != kStatusOk) *reinterpret_cast<volatile int*>(mirror) = code;
+}
+
 // ----------------------------------------------------------------------------------
 // proxy / tcgen05 fences
 // ----------------------------------------------------------------------------------

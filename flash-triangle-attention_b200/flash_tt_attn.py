@@ -43,17 +43,29 @@ _DEBUG = os.environ.get("FTA_DEBUG", "0") == "1"
 _SAVE_O_RESIDUAL = os.environ.get("FTA_SAVE_O_RESIDUAL", "1") != "0"
 _status_words = {}
 _copy_streams = {}
-_last = {"dbias_f32": None}
+_ext = None
+
+
+def _native():
+    """The torch extension that runs the passes (``_fta_torch.so``, linked against ``libfta.so``)."""
+    global _ext
+    if _ext is None:
+        _cabi.lib()  # raises with the build command where the library is missing
+        import _fta_torch
+        _fta_torch.set_save_o_residual(_SAVE_O_RESIDUAL)
+        _fta_torch.on_new_device(lambda index: _status_of(torch.device("cuda", index)))
+        _ext = _fta_torch
+    return _ext
 
 
 class _Status:
     """Per-device status word of the kernels plus a pinned host mirror of it.
 
     The kernels never trap: a bounded device-side wait that runs out writes a code to ``word`` and
-    the launch returns with unfinished outputs. After every call of this module the word is copied
-    to ``mirror`` on the stream (4 bytes, no synchronisation); the next call looks at the mirror
-    on the host before it launches anything, so a failure surfaces as an exception at most one
-    call late without the hot path ever waiting for the device."""
+    the launch returns with unfinished outputs. The kernels of ``attention()`` store a word that is not
+    zero in ``mirror`` themselves as they end; the next call looks at the mirror on the host before it
+    launches anything, so a failure surfaces as an exception at most one call late without the hot path
+    ever waiting for the device."""
 
     def __init__(self, device):
         self.word = torch.zeros(1, dtype=torch.int32, device=device)
@@ -76,6 +88,7 @@ def _status_of(device) -> _Status:
     st = _status_words.get(key)
     if st is None:
         st = _status_words[key] = _Status(device)
+        _native().set_status(device.index, st.word, st.mirror)
     return st
 
 
@@ -93,19 +106,7 @@ def check_device_status(device=None) -> None:
 
 def last_dbias_f32():
     """The float32 dBias of the most recent backward call (before rounding to the bias dtype)."""
-    return _last["dbias_f32"]
-
-
-def _dense(t: torch.Tensor) -> torch.Tensor:
-    """Inputs the kernels can address directly: unit stride in D, other strides multiples of 8
-    elements, 16-byte aligned base. Anything else is copied."""
-    ok = t.stride(-1) == 1 and all(s % 8 == 0 and s > 0 for s in t.stride()[:-1]) and t.data_ptr() % 16 == 0
-    return t if ok else t.contiguous()
-
-
-def _problem(q: torch.Tensor) -> FtaProblem:
-    B, H, L1, L2, D = q.shape
-    return FtaProblem(B, H, L1, L2, D, _cabi.FTA_BF16 if q.dtype == torch.bfloat16 else _cabi.FTA_FP16)
+    return _native().last_dbias_f32()
 
 
 def _l2p(L2: int) -> int:
@@ -113,94 +114,38 @@ def _l2p(L2: int) -> int:
 
 
 class _attention(torch.autograd.Function):
+    """The call with a process group: the same two native passes with the sum of dBias over the group
+    between the kernels and the rounding. (Without a group the autograd node is native too.)"""
+
     @staticmethod
     def forward(ctx, q, k, v, b_pw, sm_scale, group=None, key_mask=None):
-        HEAD_DIM_Q, HEAD_DIM_K, HEAD_DIM_V = q.shape[-1], k.shape[-1], v.shape[-1]
-        assert HEAD_DIM_Q == HEAD_DIM_K and HEAD_DIM_K == HEAD_DIM_V
-        assert HEAD_DIM_K in {32, 64}, "head dimension must be 32 or 64"
-        assert q.dtype == k.dtype == v.dtype == b_pw.dtype
-        assert q.dtype in (torch.float16, torch.bfloat16), "fp16 or bf16 only"
-        assert q.is_cuda, "flash_tt_attn.attention needs CUDA tensors (there is no CPU path)"
-        assert q.dim() == 5 and q.shape == k.shape == v.shape
-        B, H, L1, L2, D = q.shape
-        assert b_pw.shape == (B, H, L2, L2), "bias must be (B, H, L2, L2)"
-        assert L2 % 8 == 0, "the kernels address rows of L2 elements with 16-byte steps (attention() pads other L2)"
-
-        st = _status_of(q.device)
-        st.raise_if_set()  # an earlier call's device-side failure, seen through the host mirror
-        q, k, v, b_pw = _dense(q), _dense(k), _dense(v), _dense(b_pw)
-        L2p = _l2p(L2)
-        L = _cabi.lib()
-        prob = _problem(q)
-        o = torch.empty((B, H, L1, L2, D), dtype=q.dtype, device=q.device)
-        lse = torch.empty((3, B, H, L1, L2p), dtype=torch.float32, device=q.device)  # softmax statistics
-        # the bits of O that rounding to bf16 drops, for the backward's delta (fp16 keeps enough)
-        need_bwd = any(ctx.needs_input_grad[:4])
-        o_res = torch.empty_like(o) if (need_bwd and _SAVE_O_RESIDUAL and q.dtype == torch.bfloat16) else None
-        with torch.cuda.device(q.device):
-            stream = torch.cuda.current_stream().cuda_stream
-            bias_k = b_pw  # what the kernels read
-            if key_mask is not None or L2p != L2:
-                # Ragged L2 and / or a boolean key mask: only this bias-sized tensor is staged (whole
-                # 128-blocks, -inf on padding and masked keys); q, k, v are read in place.
-                km = None
-                if key_mask is not None:
-                    assert key_mask.dtype == torch.bool and key_mask.shape == (B, L2), "key_mask: bool (B, L2)"
-                    km = key_mask.to(device=q.device, dtype=torch.uint8).contiguous()
-                bias_k = torch.empty((B, H, L2p, L2p), dtype=q.dtype, device=q.device)
-                check(L.fta_mask_bias(prob, t4(b_pw), None if km is None else km.data_ptr(), bias_k.data_ptr(), stream),
-                      "fta_mask_bias")
-            check(L.fta_forward(prob, t5(q), t5(k), t5(v), t4(bias_k), float(sm_scale), t5(o),
-                                None if o_res is None else o_res.data_ptr(),
-                                lse.data_ptr(), st.word.data_ptr(), stream), "fta_forward")
-            st.publish()
-        if _DEBUG:
-            check_device_status(q.device)
-        ctx.save_for_backward(q, k, v, o, bias_k, lse, o_res)
+        q, k, v, bias_k, o, saved = _native().forward_pass(q, k, v, b_pw, float(sm_scale), key_mask)
+        ctx.save_for_backward(q, k, v, bias_k, o, saved)
         ctx.sm_scale = float(sm_scale)
         ctx.group = group
         return o
 
     @staticmethod
     def backward(ctx, do):
-        q, k, v, o, bias_k, lse, o_res = ctx.saved_tensors
-        assert do.dtype == q.dtype
-        do = _dense(do)
-        B, H, L1, L2, D = q.shape
-        L2p = _l2p(L2)
-        dev = q.device
-        dq = torch.empty((B, H, L1, L2, D), dtype=q.dtype, device=dev)
-        dk = torch.empty_like(dq)
-        dv = torch.empty_like(dq)
-        db = torch.empty((B, H, L2, L2), dtype=q.dtype, device=dev)
-        db32 = torch.empty((B, H, L2, L2), dtype=torch.float32, device=dev)
-        delta = torch.empty((B, H, L1, L2p), dtype=torch.float32, device=dev)
-        prob = _problem(q)
-        L = _cabi.lib()
-        ws_bytes = int(L.fta_bwd_workspace_bytes(prob))
-        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-        st = _status_of(dev)
-        st.raise_if_set()
-        status = st.word
-        sharded = ctx.group is not None
-        with torch.cuda.device(dev):
-            stream = torch.cuda.current_stream().cuda_stream
-            check(L.fta_bwd_preprocess(prob, t5(o), None if o_res is None else o_res.data_ptr(), t5(do),
-                                       delta.data_ptr(), stream), "fta_bwd_preprocess")
-            check(L.fta_backward(prob, t5(q), t5(k), t5(v), t4(bias_k), t5(do), lse.data_ptr(), delta.data_ptr(),
-                                 ctx.sm_scale, t5(dq), t5(dk), t5(dv), db32.data_ptr(),
-                                 None if sharded else db.data_ptr(), ws.data_ptr(), ws_bytes,
-                                 status.data_ptr(), stream), "fta_backward")
-            if sharded:
-                # the only collective of the path: sum the per-rank partial dBias over NVLink
-                torch.distributed.all_reduce(db32, op=torch.distributed.ReduceOp.SUM, group=ctx.group)
-                check(L.fta_dbias_cast(db32.data_ptr(), db.data_ptr(), db32.numel(), prob.dtype, stream),
-                      "fta_dbias_cast")
-            st.publish()
-        if _DEBUG:
-            check_device_status(dev)
-        _last["dbias_f32"] = db32
+        dq, dk, dv, db, db32 = _native().backward_pass(*ctx.saved_tensors, do, ctx.sm_scale, ctx.group is None)
+        if ctx.group is not None:
+            # the only collective of the path: sum the per-rank partial dBias over NVLink
+            torch.distributed.all_reduce(db32, op=torch.distributed.ReduceOp.SUM, group=ctx.group)
+            with torch.cuda.device(db.device):
+                check(_cabi.lib().fta_dbias_cast(db32.data_ptr(), db.data_ptr(), db32.numel(),
+                                                 _cabi.FTA_BF16 if db.dtype == torch.bfloat16 else _cabi.FTA_FP16,
+                                                 torch.cuda.current_stream().cuda_stream), "fta_dbias_cast")
         return dq, dk, dv, db, None, None, None
+
+
+def _call(q, k, v, b_pw, sm_scale, group, key_mask):
+    if group is not None:
+        o = _attention.apply(q, k, v, b_pw, sm_scale, group, key_mask)
+    else:
+        o = (_ext or _native()).attention(q, k, v, b_pw, float(sm_scale), key_mask)
+    if _DEBUG:
+        check_device_status(q.device)
+    return o
 
 
 def attention(q, k, v, b_pw, sm_scale, group=None, key_mask=None):
@@ -222,13 +167,13 @@ def attention(q, k, v, b_pw, sm_scale, group=None, key_mask=None):
             key_mask = key_mask.reshape(key_mask.shape[0], L2)
         key_mask = key_mask.expand(B, L2)
     if L2 % 8 == 0:
-        return _attention.apply(q, k, v, b_pw, sm_scale, group, key_mask)
+        return _call(q, k, v, b_pw, sm_scale, group, key_mask)
     pad = (L2 + 7) // 8 * 8 - L2
     F = torch.nn.functional  # F.pad is differentiable: gradients of the padding are dropped on the way back
     if key_mask is None:
         key_mask = torch.ones((B, L2), dtype=torch.bool, device=q.device)
-    out = _attention.apply(F.pad(q, (0, 0, 0, pad)), F.pad(k, (0, 0, 0, pad)), F.pad(v, (0, 0, 0, pad)),
-                           F.pad(b_pw, (0, pad, 0, pad)), sm_scale, group, F.pad(key_mask, (0, pad), value=False))
+    out = _call(F.pad(q, (0, 0, 0, pad)), F.pad(k, (0, 0, 0, pad)), F.pad(v, (0, 0, 0, pad)),
+                F.pad(b_pw, (0, pad, 0, pad)), sm_scale, group, F.pad(key_mask, (0, pad), value=False))
     return out[:, :, :, :L2]
 
 
@@ -479,7 +424,7 @@ def attention_fwd_bwd_streamed(host, sm_scale, out, block_rows=96, device=None, 
         if group is not None:
             torch.distributed.all_reduce(db32, op=torch.distributed.ReduceOp.SUM, group=group)
         out["dbias"].copy_(db32.to(b_h.dtype), non_blocking=True)
-        _last["dbias_f32"] = db32
+        _native().set_last_dbias_f32(db32)
         st.publish()
         cur.wait_stream(s_out)
         torch.cuda.synchronize(dev)
