@@ -47,14 +47,14 @@ int check_t4(const FtaTensor4* t) {
   return FTA_OK;
 }
 
-// 5-D map over (D, L2, L1, H, B), tile = 128 rows of L2 x D, swizzle = row bytes (64 or 128).
-int map5(CUtensorMap* m, const FtaProblem* p, const FtaTensor5* t) {
+// 5-D map over (D, L2, L1, H, B), tile = `box_rows` rows of L2 x D, swizzle = row bytes (64 or 128).
+int map5(CUtensorMap* m, const FtaProblem* p, const FtaTensor5* t, uint32_t box_rows = 128) {
   const uint64_t dims[5] = {static_cast<uint64_t>(p->D), static_cast<uint64_t>(p->L2),
                             static_cast<uint64_t>(p->L1), static_cast<uint64_t>(p->H),
                             static_cast<uint64_t>(p->B)};
   const uint64_t str[5] = {0, static_cast<uint64_t>(t->stride[3]) * 2, static_cast<uint64_t>(t->stride[2]) * 2,
                            static_cast<uint64_t>(t->stride[1]) * 2, static_cast<uint64_t>(t->stride[0]) * 2};
-  const uint32_t box[5] = {static_cast<uint32_t>(p->D), 128, 1, 1, 1};
+  const uint32_t box[5] = {static_cast<uint32_t>(p->D), box_rows, 1, 1, 1};
   return fta::make_tmap_16bit(m, t->ptr, 5, dims, str, box, p->D * 2) == 0 ? FTA_OK : FTA_ERR_TENSOR_MAP;
 }
 
@@ -172,18 +172,19 @@ int backward(const FtaProblem* prob, int nplanes, const FtaTensor5* q, const Fta
   bt.stride[1] = static_cast<int64_t>(l2p) * l2p;
   bt.stride[2] = l2p;
   bt.stride[3] = 1;
-  if ((rc = map5(&a.tmQ, prob, q)) || (rc = map5(&a.tmK, prob, k)) || (rc = map5(&a.tmV, prob, v)) ||
-      (rc = map5(&a.tmDO, prob, dout)) || (rc = map_bias(&a.tmBiasT, prob, &bt, 64, 128)))
+  // the backward kernel loads Q and dO by 64-query halves
+  if ((rc = map5(&a.tmQ, prob, q, 64)) || (rc = map5(&a.tmK, prob, k)) || (rc = map5(&a.tmV, prob, v)) ||
+      (rc = map5(&a.tmDO, prob, dout, 64)) || (rc = map_bias(&a.tmBiasT, prob, &bt, 64, 128)))
     return rc;
   {
-    // dq32 seen as (B*H*L1, L2, D) float32; the kernel adds 128-query x 32-column tiles into it with
+    // dq32 seen as (B*H*L1, L2, D) float32; the kernel adds 32-query x 16-column tiles into it with
     // TMA reductions (the part of a ragged last query block beyond L2 is clipped)
     const uint64_t bhi = static_cast<uint64_t>(prob->B) * prob->H * prob->L1;
     if (bhi >= (1ull << 31)) return FTA_ERR_SHAPE;  // tile coordinates are signed 32-bit
     const uint64_t dims[3] = {static_cast<uint64_t>(prob->D), static_cast<uint64_t>(prob->L2), bhi};
     const uint64_t str[3] = {0, static_cast<uint64_t>(prob->D) * 4, static_cast<uint64_t>(prob->L2) * prob->D * 4};
-    const uint32_t box[3] = {32, 128, 1};
-    if (fta::make_tmap(&a.tmDQ, 4, dq32, 3, dims, str, box, 128) != 0) return FTA_ERR_TENSOR_MAP;
+    const uint32_t dq_box[3] = {16, 32, 1}, box[3] = {32, 128, 1};
+    if (fta::make_tmap(&a.tmDQ, 4, dq32, 3, dims, str, dq_box, 64) != 0) return FTA_ERR_TENSOR_MAP;
     // the partial dBias planes, key-major: (nplanes * B*H, L2 keys, L2 queries) float32, clipped alike
     const uint64_t pdims[3] = {static_cast<uint64_t>(prob->L2), static_cast<uint64_t>(prob->L2),
                                static_cast<uint64_t>(nplanes) * prob->B * prob->H};

@@ -106,57 +106,69 @@ __device__ __forceinline__ void st_shared_volatile_u32(uint32_t addr, uint32_t v
   asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ uint32_t sm_clock() {
+  uint32_t t;
+  asm volatile("mov.u32 %0, %clock;" : "=r"(t));
+  return t;
+}
 __device__ __forceinline__ unsigned long long global_timer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
 
-// Bounded wait on an mbarrier phase. Returns false when the wait ran out or another role
-// already aborted; the caller must then skip to the tear-down.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtx& w, int site) {
-  // fast path
-  if (mbar_try_wait(bar, parity)) return true;
-  // Spin on try_wait (which itself suspends the thread for a short, bounded time). The wait
-  // gives up after `w.limit_ns` of wall-clock time, measured with the global nanosecond timer.
-  // The inner loop is nothing but the poll, so that a waiting warp takes as few issue slots as
-  // possible from the warps that share its scheduler; the abort flag is looked at once per
-  // 16 polls, the clock once per 64.
-  unsigned long long t0 = 0;
-  for (uint32_t it = 0; it < (1u << 26); ++it) {
+// Bounded wait on an mbarrier phase, executed by a full converged warp. Returns false (to all lanes alike: the
+// warp-collective tcgen05.ld / st that follow are executed by all lanes or by none) when the wait ran out; the
+// caller must then skip to the tear-down, and the roles that wait for it run out in turn.
+// Kept to a dozen instructions: a kernel inlines this at some forty places, and what lies between the instructions
+// of its loops is fetched with them (measured: a straight loop body beyond 32 KB runs at a third of its issue
+// rate). The limit is counted in SM clock cycles, two to the nanosecond.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const WaitCtx& w, int site) {
+  // one poll and one vote; try_wait suspends the thread for a short time bounded by the hardware and the hint
+  auto poll = [&] {
+    uint32_t all_ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}\n"
+        : "=r"(all_ok)
+        : "r"(bar), "r"(parity), "r"(20000u)
+        : "memory");
+    return all_ok != 0;
+  };
+  const uint32_t t0 = sm_clock();
 #pragma unroll 1
-    for (int j = 0; j < 16; ++j)
-      if (mbar_try_wait_hint(bar, parity, 20000u)) return true;
-    if (ld_shared_volatile_u32(w.abort_addr)) return false;
-    if ((it & 0x3) == 0x3) {
-      const unsigned long long now = global_timer_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > w.limit_ns) break;
-    }
+  while (!poll()) {
+    if (!__any_sync(0xffffffffu, sm_clock() - t0 > static_cast<uint32_t>(2u * w.limit_ns))) continue;
+    st_shared_volatile_u32(w.abort_addr, 1u);
+    atomicCAS(w.status, kStatusOk, kStatusWaitTimeout | site);
+    return false;
   }
-  st_shared_volatile_u32(w.abort_addr, 1u);
-  atomicCAS(w.status, kStatusOk, kStatusWaitTimeout | site);
-  return false;
+  return true;
 }
 
-// Same, executed by a full converged warp; the outcome is made warp-uniform so that the
-// warp-collective tcgen05.ld / st that follow are executed by all lanes or by none.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const WaitCtx& w, int site) {
-  // fast path: one poll and one vote, the outcome already warp-uniform
-  uint32_t all_ok;
+// One poll that never suspends the thread. What it returned some instructions ago saves a wait whose phase has
+// long completed the latency of its own poll (150 cycles and more): mbar_finish_wait.
+__device__ __forceinline__ uint32_t mbar_test_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
   asm volatile(
       "{\n\t"
-      ".reg .pred p, q;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "vote.sync.all.pred q, p, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
       "}\n"
-      : "=r"(all_ok)
+      : "=r"(ok)
       : "r"(bar), "r"(parity)
       : "memory");
-  if (all_ok) return true;
-  const bool ok = mbar_wait(bar, parity, w, site);
-  return __all_sync(0xffffffffu, ok);
+  return ok;
+}
+__device__ __forceinline__ bool mbar_finish_wait(uint32_t early, uint32_t bar, uint32_t parity, const WaitCtx& w,
+                                                 int site) {
+  if (__all_sync(0xffffffffu, early != 0)) return true;
+  return mbar_wait_warp(bar, parity, w, site);
 }
 
 // Host-visible copy of a status word (see Status in fta_kernels.h): one thread, nothing to do while the
@@ -218,8 +230,11 @@ __device__ __forceinline__ void tma_store_3d_hint(const CUtensorMap* tmap, uint3
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // the issuing thread's bulk groups have finished READING shared memory
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// all but the newest of the issuing thread's bulk groups have finished reading shared memory
-__device__ __forceinline__ void bulk_wait_read_le1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+// all but the newest kN of the issuing thread's bulk groups have finished reading shared memory / are complete
+template <int kN>
+__device__ __forceinline__ void bulk_wait_read_le() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kN) : "memory"); }
+template <int kN>
+__device__ __forceinline__ void bulk_wait_le() { asm volatile("cp.async.bulk.wait_group %0;" ::"n"(kN) : "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // bring a tile into L2 only
 __device__ __forceinline__ void tma_prefetch_l2_5d(const CUtensorMap* tmap, int c0, int c1, int c2, int c3, int c4) {
