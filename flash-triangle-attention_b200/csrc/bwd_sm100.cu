@@ -90,8 +90,8 @@ struct BwdCfg {
   static constexpr int B_ACCFULL = B_DQFREE + 2;      // per row of the group: dK / dV complete
   static constexpr int B_ACCFREE = B_ACCFULL + G;
   static constexpr int B_BOX = B_ACCFREE + G;         // dBias, per half: both boxes of a query block are parked
-  static constexpr int B_BOXFREE = B_BOX + 2;         // per spare box: it has been read
-  static constexpr int NBAR = B_BOXFREE + NX;
+  static constexpr int B_BOXFREE = B_BOX + 2;         // per half: the spare box it parked has been read
+  static constexpr int NBAR = B_BOXFREE + 2;
   static constexpr int SMEM_BYTES = OFF_BAR + NBAR * 8 + 16 + 1024;  // + tmem slot / abort flag + alignment slack
   static constexpr uint64_t SWZ = (kD == 32) ? kSwz64 : kSwz128;
   static constexpr uint32_t ROW_B = kD * 2;
@@ -188,8 +188,8 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       mbar_init(bar(C::B_XFULL + i), 1);
       mbar_init(bar(C::B_UFULL + i), 4);  // one arrive per warp of the half
       mbar_init(bar(C::B_BOX + i), 4);
+      mbar_init(bar(C::B_BOXFREE + i), 1);
     }
-    for (int i = 0; i < C::NX; ++i) mbar_init(bar(C::B_BOXFREE + i), 1);
     mbar_fence_init();
   }
   if (threadIdx.x < 64) reinterpret_cast<uint32_t*>(sZero)[threadIdx.x] = 0u;
@@ -442,7 +442,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
               bulk_wait_read_le<1>();
               mbar_arrive(bar(C::B_BIASEMPTY + bs));
               bulk_wait_read_all();
-              mbar_arrive(bar(C::B_BOXFREE + x));
+              mbar_arrive(bar(C::B_BOXFREE + hf));
             }
             __syncwarp();
           }
@@ -667,10 +667,12 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         if (!ok) break;
         // The sums of this query block as two boxes (128 key rows x 32 queries, 128-byte swizzle): one in the block's
         // half bias stage (this thread's row of it, whose bias values nobody else reads), one in the spare box,
-        // whose previous contents left while the block was worked on.
-        const int use = C::NX == 2 ? nb : 2 * nb + hf;  // earlier uses of the spare box
-        if (use > 0) {
-          ok = mbar_wait_warp(bar(C::B_BOXFREE + (hf & (C::NX - 1))), (use - 1) & 1, w, 0x4b);
+        // whose previous contents left while the block was worked on. With one spare box for both halves those are
+        // the other half's; a barrier per half, each waited for once per block, never runs a phase ahead.
+        const int by = C::NX == 2 ? hf : hf ^ 1;                         // who parked there last
+        const int use = (C::NX == 2 || hf == 0) ? nb - 1 : nb;           // in which block
+        if (use >= 0) {
+          ok = mbar_wait_warp(bar(C::B_BOXFREE + by), use & 1, w, 0x4b);
           if (!ok) break;
         }
 #pragma unroll
