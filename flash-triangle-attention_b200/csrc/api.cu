@@ -19,10 +19,12 @@ int cuda_fail(int e) { return cuda_fail(static_cast<cudaError_t>(e)); }
 
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
-int check_problem(const FtaProblem* p) {
+// The C ABI takes L2 in multiples of 8 (its dBias buffers and biases have rows of L2 elements, read and written
+// 16 bytes at a time); the native entry points stage the bias and take any L2.
+int check_problem(const FtaProblem* p, bool any_l2 = false) {
   if (!p) return FTA_ERR_NULL;
   if (p->B <= 0 || p->H <= 0 || p->L1 <= 0 || p->L2 <= 0) return FTA_ERR_SHAPE;
-  if (p->L2 % 8 != 0) return FTA_ERR_SHAPE;
+  if (!any_l2 && p->L2 % 8 != 0) return FTA_ERR_SHAPE;
   if (p->D != 32 && p->D != 64) return FTA_ERR_HEAD_DIM;
   if (p->dtype != FTA_FP16 && p->dtype != FTA_BF16) return FTA_ERR_DTYPE;
   if (static_cast<long long>(p->B) * p->H > 65535) return FTA_ERR_TOO_LARGE;
@@ -78,7 +80,10 @@ int map_bias(CUtensorMap* m, const FtaProblem* p, const FtaTensor4* t, int box_k
 
 size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
-size_t plane_bytes(const FtaProblem* p) { return static_cast<size_t>(p->B) * p->H * p->L2 * p->L2 * sizeof(float); }
+size_t plane_pitch(const FtaProblem* p) { return (static_cast<size_t>(p->L2) + 7) / 8 * 8; }  // elements of a plane row
+size_t plane_bytes(const FtaProblem* p) {
+  return static_cast<size_t>(p->B) * p->H * p->L2 * plane_pitch(p) * sizeof(float);
+}
 size_t dq32_bytes(const FtaProblem* p) {
   return static_cast<size_t>(p->B) * p->H * p->L1 * p->L2 * p->D * sizeof(float);
 }
@@ -93,7 +98,7 @@ int plan_planes(const FtaProblem* p) { return fta::bwd_num_planes(p->B, p->H, p-
 int forward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
             const FtaTensor4* bias, float sm_scale, const FtaTensor5* o, void* o_resid, float* lse, fta::Status status,
             cudaStream_t stream) {
-  int rc = check_problem(prob);
+  int rc = check_problem(prob, true);
   if (rc) return rc;
   if ((rc = check_t5(q)) || (rc = check_t5(k)) || (rc = check_t5(v)) || (rc = check_t5(o)) || (rc = check_t4(bias)))
     return rc;
@@ -119,32 +124,32 @@ int forward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* k, co
   return FTA_OK;
 }
 
-int preprocess(const FtaProblem* prob, const FtaTensor5* o, const void* o_resid, const FtaTensor5* dout, float* delta,
-               cudaStream_t stream) {
-  int rc = check_problem(prob);
-  if (rc) return rc;
+int fill_pre(fta::PreArgs* a, const FtaProblem* prob, const FtaTensor5* o, const void* o_resid, const FtaTensor5* dout,
+             float* delta) {
+  int rc;
   if ((rc = check_t5(o)) || (rc = check_t5(dout))) return rc;
   if (!delta) return FTA_ERR_NULL;
   if (!aligned16(o_resid)) return FTA_ERR_ALIGN;
-  long long so[4], sd[4];
+  a->o = o->ptr;
+  a->o_resid = o_resid;
+  a->dout = dout->ptr;
+  a->delta = delta;
+  a->delta_pitch = padded_l2(prob);
   for (int i = 0; i < 4; ++i) {
-    so[i] = o->stride[i];
-    sd[i] = dout->stride[i];
+    a->so[i] = o->stride[i];
+    a->sdo[i] = dout->stride[i];
   }
-  const int l2p = padded_l2(prob);
-  if (l2p != prob->L2) {
-    // the entries of queries past L2 (whole 128-blocks are read by the backward kernel) must be finite
-    const cudaError_t e = cudaMemsetAsync(
-        delta, 0, sizeof(float) * static_cast<size_t>(prob->B) * prob->H * prob->L1 * l2p, stream);
-    if (e != cudaSuccess) return cuda_fail(e);
-  }
-  if (const int e = fta::launch_preprocess(o->ptr, o_resid, so, dout->ptr, sd, delta, l2p, prob->B, prob->H, prob->L1,
-                                           prob->L2, prob->D, prob->dtype == FTA_BF16, stream))
-    return cuda_fail(e);
+  a->B = prob->B;
+  a->H = prob->H;
+  a->L1 = prob->L1;
+  a->L2 = prob->L2;
+  a->D = prob->D;
+  a->bf16 = prob->dtype == FTA_BF16;
   return FTA_OK;
 }
 
-int backward(const FtaProblem* prob, int nplanes, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
+// `pre`: also run the preprocess it describes, in the launch of the prologue (nullptr: delta is there already)
+int backward(const FtaProblem* prob, int nplanes, const fta::PreArgs* pre, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
              const FtaTensor4* bias, const FtaTensor5* dout, const float* lse, const float* delta, float sm_scale,
              const FtaTensor5* dq, const FtaTensor5* dk, const FtaTensor5* dv, float* dbias_f32, void* dbias_cast,
              void* workspace, size_t have_bytes, fta::Status status, cudaStream_t st) {
@@ -188,7 +193,8 @@ int backward(const FtaProblem* prob, int nplanes, const FtaTensor5* q, const Fta
     // the partial dBias planes, key-major: (nplanes * B*H, L2 keys, L2 queries) float32, clipped alike
     const uint64_t pdims[3] = {static_cast<uint64_t>(prob->L2), static_cast<uint64_t>(prob->L2),
                                static_cast<uint64_t>(nplanes) * prob->B * prob->H};
-    const uint64_t pstr[3] = {0, static_cast<uint64_t>(prob->L2) * 4, static_cast<uint64_t>(prob->L2) * prob->L2 * 4};
+    const uint64_t pitch = plane_pitch(prob) * 4;
+    const uint64_t pstr[3] = {0, pitch, prob->L2 * pitch};
     if (fta::make_tmap(&a.tmPlane, 4, planes, 3, pdims, pstr, box, 128) != 0) return FTA_ERR_TENSOR_MAP;
   }
   a.lse = lse;
@@ -215,7 +221,7 @@ int backward(const FtaProblem* prob, int nplanes, const FtaTensor5* q, const Fta
   long long sb[4];
   for (int i = 0; i < 4; ++i) sb[i] = bias->stride[i];
   if (const int e = fta::launch_bwd_prologue(bias->ptr, sb, bias_t, prob->B, prob->H, l2p, dq32,
-                                             static_cast<long long>(rows) * prob->D, st))
+                                             static_cast<long long>(rows) * prob->D, pre, st))
     return cuda_fail(e);
   if (g_prof_start) cudaEventRecord(g_prof_start, st);
   if (const int e = fta::launch_bwd(a, st)) return cuda_fail(e);
@@ -239,8 +245,20 @@ int native_forward(const FtaProblem& prob, const FtaTensor5& q, const FtaTensor5
   return forward(&prob, &q, &k, &v, &bias, sm_scale, &o, o_resid, lse, {status.word, status.mirror}, stream);
 }
 
+int native_mask_bias(const FtaProblem& prob, const FtaTensor4& bias, const uint8_t* key_mask, void* out,
+                     cudaStream_t stream) {
+  if (const int rc = check_problem(&prob, true)) return rc;
+  if (!bias.ptr || !out) return FTA_ERR_NULL;
+  if (!aligned16(out)) return FTA_ERR_ALIGN;
+  const long long sb[4] = {bias.stride[0], bias.stride[1], bias.stride[2], bias.stride[3]};
+  if (const int e = fta::launch_mask_bias(bias.ptr, sb, key_mask, out, prob.B, prob.H, prob.L2, padded_l2(&prob),
+                                          prob.dtype == FTA_BF16, stream))
+    return cuda_fail(e);
+  return FTA_OK;
+}
+
 int native_backward_plan(const FtaProblem& prob, BackwardPlan* plan) {
-  if (const int rc = check_problem(&prob)) return rc;
+  if (const int rc = check_problem(&prob, true)) return rc;
   plan->nplanes = plan_planes(&prob);
   plan->workspace_bytes = workspace_bytes(&prob, plan->nplanes);
   plan->delta_bytes = sizeof(float) * static_cast<size_t>(prob.B) * prob.H * prob.L1 * padded_l2(&prob);
@@ -253,8 +271,9 @@ int native_backward(const FtaProblem& prob, const BackwardPlan& plan, const FtaT
                     const FtaTensor5& dk, const FtaTensor5& dv, float* dbias_f32, void* dbias_cast, void* workspace,
                     StatusPair status, cudaStream_t stream) {
   float* delta = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + plan.workspace_bytes);
-  if (const int rc = preprocess(&prob, &o, o_resid, &dout, delta, stream)) return rc;
-  return backward(&prob, plan.nplanes, &q, &k, &v, &bias, &dout, lse, delta, sm_scale, &dq, &dk, &dv, dbias_f32,
+  fta::PreArgs pre;
+  if (const int rc = fill_pre(&pre, &prob, &o, o_resid, &dout, delta)) return rc;
+  return backward(&prob, plan.nplanes, &pre, &q, &k, &v, &bias, &dout, lse, delta, sm_scale, &dq, &dk, &dv, dbias_f32,
                   dbias_cast, workspace, plan.workspace_bytes, {status.word, status.mirror}, stream);
 }
 
@@ -294,7 +313,11 @@ int fta_forward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* k
 
 int fta_bwd_preprocess(const FtaProblem* prob, const FtaTensor5* o, const void* o_resid, const FtaTensor5* dout,
                        float* delta, void* stream) {
-  return preprocess(prob, o, o_resid, dout, delta, static_cast<cudaStream_t>(stream));
+  fta::PreArgs a;
+  if (const int rc = check_problem(prob)) return rc;
+  if (const int rc = fill_pre(&a, prob, o, o_resid, dout, delta)) return rc;
+  if (const int e = fta::launch_preprocess(a, static_cast<cudaStream_t>(stream))) return cuda_fail(e);
+  return FTA_OK;
 }
 
 int fta_mask_bias(const FtaProblem* prob, const FtaTensor4* bias, const uint8_t* key_mask, void* out, void* stream) {
@@ -323,7 +346,7 @@ int fta_backward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* 
                  float* dbias_f32, void* dbias_cast, void* workspace, size_t workspace_bytes, int32_t* status,
                  void* stream) {
   if (const int rc = check_problem(prob)) return rc;
-  return backward(prob, plan_planes(prob), q, k, v, bias, dout, lse, delta, sm_scale, dq, dk, dv, dbias_f32, dbias_cast,
+  return backward(prob, plan_planes(prob), nullptr, q, k, v, bias, dout, lse, delta, sm_scale, dq, dk, dv, dbias_f32, dbias_cast,
                   workspace, workspace_bytes, {status, nullptr}, static_cast<cudaStream_t>(stream));
 }
 

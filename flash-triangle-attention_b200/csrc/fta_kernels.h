@@ -94,25 +94,34 @@ int launch_bwd(const BwdArgs& a, cudaStream_t stream);
 int bwd_rows_per_cta(int D);
 int bwd_num_planes(int B, int H, int L1, int L2, int D, int sms);
 
-// delta[(b,h,i), j] = sum_d (O[.,d] + R[.,d]) * dO[.,d]; `o_resid` (R, strides of O) may be nullptr;
-// `delta_pitch` = elements between rows (b,h,i) of delta (L2 rounded up to 128)
-int launch_preprocess(const void* o, const void* o_resid, const long long so[4], const void* dout,
-                      const long long sdo[4], float* delta, int delta_pitch, int B, int H, int L1, int L2, int D,
-                      bool bf16, cudaStream_t stream);
+// delta[(b,h,i), j] = sum_d (O[.,d] + R[.,d]) * dO[.,d] for j < L2 and 0 up to `delta_pitch` (elements between rows
+// (b,h,i) of delta: L2 rounded up to 128; the backward kernel reads whole 128-blocks)
+struct PreArgs {
+  const void* o;
+  const void* o_resid;  // R, strides of O; may be nullptr
+  const void* dout;
+  float* delta;
+  int delta_pitch, B, H, L1, L2, D;
+  bool bf16;
+  long long so[4], sdo[4];  // element strides of O, dO over (B, H, L1, L2)
+};
+int launch_preprocess(const PreArgs& a, cudaStream_t stream);
 
 // out[b][h][q][k], (B, H, L2p, L2p) contiguous: the bias where q, k < L2 and the key is kept by
 // `key_mask` ((B, L2) bytes, non-zero = keep; nullptr = keep all), -inf for every other key, 0 for
-// the kept keys of the padding queries q >= L2
+// the kept keys of the padding queries q >= L2. `sb`: element strides of the bias; 16-byte loads where they, L2
+// and the pointers allow it, single elements otherwise
 int launch_mask_bias(const void* bias, const long long sb[4], const uint8_t* key_mask, void* out, int B, int H, int L2,
                      int L2p, bool bf16, cudaStream_t stream);
 
 // Backward prologue, one launch: bias_t[bh][k][q] = bias[b][h][q][k] (16-bit elements; `sb` = element
-// strides of the bias) and zero-fill of the float32 dQ accumulator (`dq_elems` floats, a multiple of 4)
+// strides of the bias) and zero-fill of the float32 dQ accumulator (`dq_elems` floats, a multiple of 4); with `pre`
+// the preprocess too (three independent streams that share the launch)
 int launch_bwd_prologue(const void* bias, const long long sb[4], void* bias_t, int B, int H, int L2, float* dq32,
-                        long long dq_elems, cudaStream_t stream);
+                        long long dq_elems, const PreArgs* pre, cudaStream_t stream);
 
 // Backward epilogue, one launch: dq[row, d] = (dtype)(scale * dq32[row, d]) and, for the KEY-MAJOR
-// planes the backward kernel writes, (nplanes, B*H, key, query):
+// planes the backward kernel writes, (nplanes, B*H, key, query) with rows of L2 rounded up to 8 elements:
 // dbias_f32[bh][query][key] = sum_p planes[p][bh][key][query] in plane order, optional rounded copy
 int launch_bwd_epilogue(const float* dq32, void* dq, const long long sdq[4], int B, int H, int L1, int L2, int D,
                         float scale, const float* planes, int nplanes, float* dbias_f32, void* dbias_cast, bool bf16,

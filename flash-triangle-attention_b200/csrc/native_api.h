@@ -1,7 +1,8 @@
 // C++ entry points of libfta.so for the torch extension that ships beside it (torch_binding.cpp). They run
 // the same validation and launches as the C ABI (include/fta.h); what they add is what a caller that owns
-// both passes can use: a host mirror of the status word, a forward pass without statistics, and the whole
-// backward pass (preprocess included) as one call planned once.
+// both passes can use: any L2 (with a staged bias; the C ABI takes multiples of 8), a host mirror of the status
+// word, a forward pass without statistics, and the whole backward pass (preprocess included) as one call
+// planned once.
 #pragma once
 
 #include "../../include/fta.h"
@@ -22,6 +23,10 @@ struct StatusPair {
 FTA_NATIVE int native_forward(const FtaProblem& prob, const FtaTensor5& q, const FtaTensor5& k, const FtaTensor5& v,
                               const FtaTensor4& bias, float sm_scale, const FtaTensor5& o, void* o_resid, float* lse,
                               StatusPair status, cudaStream_t stream);
+
+// fta_mask_bias for any L2, any strides and any alignment of the bias and the mask
+FTA_NATIVE int native_mask_bias(const FtaProblem& prob, const FtaTensor4& bias, const uint8_t* key_mask, void* out,
+                                cudaStream_t stream);
 
 // What fta_backward and fta_bwd_preprocess need in scratch memory for `prob`, planned once per call
 struct BackwardPlan {

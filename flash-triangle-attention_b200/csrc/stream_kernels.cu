@@ -5,8 +5,8 @@
 //                   _attn_bwd_preprocess, flash_tt_attn.py:266-288; R is the optional rounding
 //                   residual of O written by the forward pass)
 //  bwd_prologue   : key-major copy of the pair bias for the backward kernel + zero-fill of the
-//                   float32 dQ accumulator, one launch (the reference zero-fills its dBias buffer
-//                   instead, flash_tt_attn.py:613)
+//                   float32 dQ accumulator + the preprocess (where the caller runs the whole pass), one
+//                   launch (the reference zero-fills its dBias buffer instead, flash_tt_attn.py:613)
 //  bwd_epilogue   : dQ = (dtype)(sm_scale * dQ_f32) (the scaling of flash_tt_attn.py:430, 549) and
 //                   dBias = sum over the partial planes in plane order, transposed back to
 //                   (query, key), plus the rounded copy (replaces the fp16 atomics into a zeroed
@@ -70,18 +70,17 @@ __device__ __forceinline__ long long strided_row_offset(long long row, int H, in
 // One thread per 8 elements; D/8 adjacent lanes share a row and reduce with shuffles.
 // kDense: both tensors are contiguous, so a row's offset is row * D and the index needs no
 // division (the strided form spends more instructions on 64-bit divisions than on the data).
+// `block` of `nblocks`: this block's share of the rows.
 template <int kD, bool kBf16, bool kDense, bool kResid>
-__global__ void __launch_bounds__(256) preprocess_kernel(const uint16_t* __restrict__ o,
-                                                         const uint16_t* __restrict__ o_resid,
-                                                         const uint16_t* __restrict__ dout,
-                                                         float* __restrict__ delta, int delta_pitch,
-                                                         long long rows, int H, int L1, int L2, long long so_b,
-                                                         long long so_h, long long so_i, long long so_j,
-                                                         long long sd_b, long long sd_h, long long sd_i,
-                                                         long long sd_j) {
+__device__ __forceinline__ void preprocess_rows(const PreArgs& a, int block, int nblocks) {
   constexpr int LPR = kD / 8;  // lanes per row
-  const long long nthreads = static_cast<long long>(gridDim.x) * blockDim.x;
-  const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const uint16_t* __restrict__ o = static_cast<const uint16_t*>(a.o);
+  const uint16_t* __restrict__ o_resid = static_cast<const uint16_t*>(a.o_resid);
+  const uint16_t* __restrict__ dout = static_cast<const uint16_t*>(a.dout);
+  const int L2 = a.L2;
+  const long long rows = static_cast<long long>(a.B) * a.H * a.L1 * L2;
+  const long long nthreads = static_cast<long long>(nblocks) * blockDim.x;
+  const long long tid = static_cast<long long>(block) * blockDim.x + threadIdx.x;
   const long long total = (rows * LPR + 31) / 32 * 32;  // keep warps converged for the shuffles
   for (long long idx = tid; idx < total; idx += nthreads) {
     const long long row = idx / LPR;
@@ -92,8 +91,8 @@ __global__ void __launch_bounds__(256) preprocess_kernel(const uint16_t* __restr
       if constexpr (kDense) {
         oo = od = row * kD + part * 8;
       } else {
-        oo = strided_row_offset(row, H, L1, L2, so_b, so_h, so_i, so_j) + part * 8;
-        od = strided_row_offset(row, H, L1, L2, sd_b, sd_h, sd_i, sd_j) + part * 8;
+        oo = strided_row_offset(row, a.H, a.L1, L2, a.so[0], a.so[1], a.so[2], a.so[3]) + part * 8;
+        od = strided_row_offset(row, a.H, a.L1, L2, a.sdo[0], a.sdo[1], a.sdo[2], a.sdo[3]) + part * 8;
       }
       const uint4 ov = __ldg(reinterpret_cast<const uint4*>(o + oo));
       const uint4 dv = __ldg(reinterpret_cast<const uint4*>(dout + od));
@@ -106,9 +105,23 @@ __global__ void __launch_bounds__(256) preprocess_kernel(const uint16_t* __restr
     }
 #pragma unroll
     for (int off = LPR / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    // rows of delta are `delta_pitch` apart (L2 rounded up to 128; equal to L2 in the dense case)
-    if (part == 0 && row < rows) delta[delta_pitch == L2 ? row : (row / L2) * delta_pitch + row % L2] = s;
+    if (part == 0 && row < rows) {
+      if (a.delta_pitch == L2) {
+        a.delta[row] = s;
+      } else {  // a ragged row's padding is zeroed by the rows themselves
+        const long long r = row / L2;
+        const int j = static_cast<int>(row - r * L2);
+        float* d = a.delta + r * a.delta_pitch;
+        d[j] = s;
+        for (int z = L2 + j; z < a.delta_pitch; z += L2) d[z] = 0.f;
+      }
+    }
   }
+}
+
+template <int kD, bool kBf16, bool kDense, bool kResid>
+__global__ void __launch_bounds__(256) preprocess_kernel(const PreArgs a) {
+  preprocess_rows<kD, kBf16, kDense, kResid>(a, blockIdx.x, gridDim.x);
 }
 
 template <bool kBf16>
@@ -346,10 +359,11 @@ __global__ void __launch_bounds__(64) peers_wait_kernel(const int* done_words, i
 }
 
 // Padded, masked copy of the pair bias for problems whose L2 is not a multiple of 128 and / or that
-// drop keys with a boolean mask: out (B*H, L2p, L2p), 8 elements (16 bytes) per thread.
-template <bool kBf16>
+// drop keys with a boolean mask: out (B*H, L2p, L2p), 8 elements (16 bytes) per thread. kVec: the source is read
+// 16 bytes at a time too (L2 and the strides multiples of 8, aligned pointers); otherwise element by element.
+template <bool kBf16, bool kVec>
 __global__ void __launch_bounds__(256) mask_bias_kernel(const uint16_t* __restrict__ bias, long long s_b, long long s_h,
-                                                        long long s_q, const uint8_t* __restrict__ key_mask,
+                                                        long long s_q, long long s_k, const uint8_t* __restrict__ key_mask,
                                                         uint16_t* __restrict__ out, int BH, int H, int L2, int L2p) {
   constexpr uint32_t NEG_INF = kBf16 ? 0xFF80u : 0xFC00u;
   const int vec_per_row = L2p / 8;
@@ -364,6 +378,16 @@ __global__ void __launch_bounds__(256) mask_bias_kernel(const uint16_t* __restri
     uint32_t w[4] = {0u, 0u, 0u, 0u};
     if (k8 >= L2) {
       w[0] = w[1] = w[2] = w[3] = NEG_INF | (NEG_INF << 16);  // padding keys: never attended
+    } else if constexpr (!kVec) {
+      const uint16_t* src = bias + b * s_b + h * s_h + q * s_q;
+      const uint8_t* km = key_mask ? key_mask + static_cast<long long>(b) * L2 : nullptr;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int k = k8 + e;
+        uint32_t x = NEG_INF;
+        if (k < L2 && (!km || km[k])) x = q < L2 ? src[k * s_k] : 0u;  // padding queries see a zero bias on the real keys
+        w[e >> 1] |= x << ((e & 1) * 16);
+      }
     } else {
       uint4 v = make_uint4(0u, 0u, 0u, 0u);  // padding queries see a zero bias on the real keys
       if (q < L2) v = __ldg(reinterpret_cast<const uint4*>(bias + b * s_b + h * s_h + q * s_q + k8));
@@ -386,15 +410,24 @@ __global__ void __launch_bounds__(256) mask_bias_kernel(const uint16_t* __restri
 // Backward prologue. Blocks [0, tr_blocks): out[bh][k][q] = bias[b][h][q][k] (16-bit elements, 64 x 64
 // tiles through shared memory, 16-byte global accesses on both sides). Remaining blocks: zero-fill
 // of the float32 dQ accumulator, 16 bytes per thread, grid-stride.
+// The last `pre_blocks` blocks run the preprocess (kPre; template arguments as there).
 // ------------------------------------------------------------------------------------------------
+template <bool kPre, int kD, bool kBf16, bool kDense, bool kResid>
 __global__ void __launch_bounds__(256) bwd_prologue_kernel(const uint16_t* __restrict__ bias,
                                                            uint16_t* __restrict__ bias_t, int BH, int H, int L2,
                                                            long long s_b, long long s_h, long long s_q,
                                                            int tr_blocks, float4* __restrict__ dq32,
-                                                           long long dq_vec) {
+                                                           long long dq_vec, int pre_blocks, const PreArgs pre) {
   __shared__ uint32_t tile[64][33];  // [query][key pair]; odd pitch in words
+  const int first_pre = static_cast<int>(gridDim.x) - pre_blocks;
+  if constexpr (kPre) {
+    if (static_cast<int>(blockIdx.x) >= first_pre) {
+      preprocess_rows<kD, kBf16, kDense, kResid>(pre, blockIdx.x - first_pre, pre_blocks);
+      return;
+    }
+  }
   if (static_cast<int>(blockIdx.x) >= tr_blocks) {
-    const long long nthreads = static_cast<long long>(gridDim.x - tr_blocks) * blockDim.x;
+    const long long nthreads = static_cast<long long>(first_pre - tr_blocks) * blockDim.x;
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
     for (long long v = static_cast<long long>(blockIdx.x - tr_blocks) * blockDim.x + threadIdx.x; v < dq_vec;
          v += nthreads)
@@ -442,10 +475,11 @@ __global__ void __launch_bounds__(256) bwd_prologue_kernel(const uint16_t* __res
 
 // ------------------------------------------------------------------------------------------------
 // Backward epilogue. Blocks [0, dq_blocks): dq = dtype(scale * dq32), 8 elements per thread,
-// grid-stride. Remaining blocks: one 64 (key) x 64 (query) tile of dBias each - the key-major
-// planes (p, bh, key, query) summed in plane order in registers (float4 loads along the query
-// axis), transposed through shared memory, written as (bh, query, key) float32 and 16-bit with
-// 16-byte stores along the key axis. Fixed order everywhere: bit-reproducible.
+// grid-stride. Remaining blocks: one 32 (key) x 32 (query) tile of dBias each - the key-major
+// planes (p, bh, key, query) summed in plane order in registers (one float4 along the query axis per
+// thread and plane), transposed through shared memory, written as (bh, query, key) float32 and 16-bit.
+// Fixed order everywhere: bit-reproducible. The planes of a small problem are many (one per row block) and its
+// tiles few, a chain of dependent memory latencies: hence the small tile and eight planes in flight.
 // ------------------------------------------------------------------------------------------------
 template <int kD, bool kBf16, bool kDense>
 __global__ void __launch_bounds__(256) bwd_epilogue_kernel(const float* __restrict__ dq32, uint16_t* __restrict__ dq,
@@ -454,7 +488,7 @@ __global__ void __launch_bounds__(256) bwd_epilogue_kernel(const float* __restri
                                                            int dq_blocks, const float* __restrict__ planes, int nplanes,
                                                            int BH, float* __restrict__ out_f32,
                                                            uint16_t* __restrict__ out_cast, Status status) {
-  __shared__ float tile[64][65];  // [key][query]
+  __shared__ float tile[32][33];  // [key][query]
   if (blockIdx.x == 0 && threadIdx.x == 0) publish_status(status.word, status.mirror);
   if (static_cast<int>(blockIdx.x) < dq_blocks) {
     constexpr int LPR = kD / 8;
@@ -478,86 +512,54 @@ __global__ void __launch_bounds__(256) bwd_epilogue_kernel(const float* __restri
     }
     return;
   }
-  const int tiles = (L2 + 63) / 64;  // L2 is a multiple of 8: an 8-key / 4-query vector is inside or outside as a whole
+  const int tiles = (L2 + 31) / 32;
   int t = blockIdx.x - dq_blocks;
-  const int q0 = (t % tiles) * 64;
+  const int q0 = (t % tiles) * 32;
   t /= tiles;
-  const int k0 = (t % tiles) * 64;
+  const int k0 = (t % tiles) * 32;
   const int bh = t / tiles;
-  const long long plane_stride = static_cast<long long>(BH) * L2 * L2;
-  // read: thread -> key rows kr, kr + 16, kr + 32, kr + 48, four queries at qc
-  const int kr = threadIdx.x >> 4, qc = (threadIdx.x & 15) * 4;
-  const float* src = planes + (static_cast<long long>(bh) * L2 + k0 + kr) * L2 + q0 + qc;
-  float4 acc[4];
+  const int pitch = (L2 + 7) & ~7;
+  const long long plane_stride = static_cast<long long>(BH) * L2 * pitch;
+  const int kr = threadIdx.x >> 3, qc = (threadIdx.x & 7) * 4;  // this thread's key row, its four queries
+  if (k0 + kr < L2 && q0 + qc < L2) {
+    const float* src = planes + (static_cast<long long>(bh) * L2 + k0 + kr) * pitch + q0 + qc;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    constexpr int U = 8;
+    for (int p0 = 0; p0 < nplanes; p0 += U) {
+      float4 x[U];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  const bool q_in = q0 + qc < L2;
-  // planes added in index order (bit-reproducible); the loads of four planes are in flight together:
-  // with one head per GPU there are only (L2/64)^2 of these blocks and up to 24 planes each, a chain
-  // of dependent memory latencies when the planes are read one at a time
-  auto load = [&](int pl, int i) {
-    return __ldg(reinterpret_cast<const float4*>(src + static_cast<long long>(pl) * plane_stride +
-                                                 static_cast<long long>(16 * i) * L2));
-  };
-  int pl = 0;
-  for (; pl + 4 <= nplanes; pl += 4) {
-    float4 x[4][4];
+      for (int u = 0; u < U; ++u)
+        if (p0 + u < nplanes) x[u] = __ldg(reinterpret_cast<const float4*>(src + (p0 + u) * plane_stride));
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        x[u][i] = (q_in && k0 + kr + 16 * i < L2) ? load(pl + u, i) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        acc[i].x += x[u][i].x;
-        acc[i].y += x[u][i].y;
-        acc[i].z += x[u][i].z;
-        acc[i].w += x[u][i].w;
+      for (int u = 0; u < U; ++u) {
+        if (p0 + u >= nplanes) break;
+        acc.x += x[u].x;
+        acc.y += x[u].y;
+        acc.z += x[u].z;
+        acc.w += x[u].w;
       }
-  }
-  for (; pl < nplanes; ++pl) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (!q_in || k0 + kr + 16 * i >= L2) continue;
-      const float4 x = load(pl, i);
-      acc[i].x += x.x;
-      acc[i].y += x.y;
-      acc[i].z += x.z;
-      acc[i].w += x.w;
     }
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float* trow = &tile[kr + 16 * i][qc];
-    trow[0] = acc[i].x;
-    trow[1] = acc[i].y;
-    trow[2] = acc[i].z;
-    trow[3] = acc[i].w;
+    tile[kr][qc] = acc.x;
+    tile[kr][qc + 1] = acc.y;
+    tile[kr][qc + 2] = acc.z;
+    tile[kr][qc + 3] = acc.w;
   }
   __syncthreads();
-  // write: 64 queries x 8 groups of 8 keys = 512 items, two per thread
+  // write: 32 queries x 8 groups of 4 keys
+  const int q = threadIdx.x >> 3, k4 = (threadIdx.x & 7) * 4;
+  if (q0 + q >= L2 || k0 + k4 >= L2) return;
+  const float v[4] = {tile[k4][q], tile[k4 + 1][q], tile[k4 + 2][q], tile[k4 + 3][q]};
+  const long long o = (static_cast<long long>(bh) * L2 + q0 + q) * L2 + k0 + k4;
+  const uint2 pk = make_uint2(pack2<kBf16>(v[0], v[1]), pack2<kBf16>(v[2], v[3]));
+  if ((L2 & 3) == 0) {
+    if (out_f32) *reinterpret_cast<float4*>(out_f32 + o) = make_float4(v[0], v[1], v[2], v[3]);
+    if (out_cast) *reinterpret_cast<uint2*>(out_cast + o) = pk;
+  } else {
 #pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int c = threadIdx.x + it * 256;
-    const int q = c >> 3, k8 = (c & 7) * 8;
-    if (q0 + q >= L2 || k0 + k8 >= L2) continue;
-    float v[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = tile[k8 + e][q];
-    const long long o = (static_cast<long long>(bh) * L2 + q0 + q) * L2 + k0 + k8;
-    if (out_f32) {
-      *reinterpret_cast<float4*>(out_f32 + o) = make_float4(v[0], v[1], v[2], v[3]);
-      *reinterpret_cast<float4*>(out_f32 + o + 4) = make_float4(v[4], v[5], v[6], v[7]);
-    }
-    if (out_cast) {
-      uint4 pk;
-      pk.x = pack2<kBf16>(v[0], v[1]);
-      pk.y = pack2<kBf16>(v[2], v[3]);
-      pk.z = pack2<kBf16>(v[4], v[5]);
-      pk.w = pack2<kBf16>(v[6], v[7]);
-      *reinterpret_cast<uint4*>(out_cast + o) = pk;
+    for (int e = 0; e < 4; ++e) {
+      if (k0 + k4 + e >= L2) break;
+      if (out_f32) out_f32[o + e] = v[e];
+      if (out_cast) out_cast[o + e] = static_cast<uint16_t>((e < 2 ? pk.x : pk.y) >> ((e & 1) * 16));
     }
   }
 }
@@ -577,61 +579,71 @@ bool is_dense(const long long s4[4], int H, int L1, int L2, int D) {
 
 }  // namespace
 
-int launch_preprocess(const void* o, const void* o_resid, const long long so[4], const void* dout,
-                      const long long sdo[4], float* delta, int delta_pitch, int B, int H, int L1, int L2, int D,
-                      bool bf16, cudaStream_t stream) {
-  const long long rows = static_cast<long long>(B) * H * L1 * L2;
-  const int grid = grid_for(rows * (D / 8), 256);
-  const uint16_t* op = static_cast<const uint16_t*>(o);
-  const uint16_t* rp = static_cast<const uint16_t*>(o_resid);
-  const uint16_t* dp = static_cast<const uint16_t*>(dout);
-  const bool dense = is_dense(so, H, L1, L2, D) && is_dense(sdo, H, L1, L2, D);
-  auto go = [&](auto kern) {
-    kern<<<grid, 256, 0, stream>>>(op, rp, dp, delta, delta_pitch, rows, H, L1, L2, so[0], so[1], so[2], so[3],
-                                   sdo[0], sdo[1], sdo[2], sdo[3]);
-  };
-  auto pick = [&](auto d_tag, auto bf_tag) {
-    constexpr int DD = decltype(d_tag)::value;
-    constexpr bool BF = decltype(bf_tag)::value;
-    if (dense) {
-      if (rp) go(preprocess_kernel<DD, BF, true, true>);
-      else go(preprocess_kernel<DD, BF, true, false>);
-    } else {
-      if (rp) go(preprocess_kernel<DD, BF, false, true>);
-      else go(preprocess_kernel<DD, BF, false, false>);
-    }
+namespace {
+// calls f.operator()<D, bf16, dense, residual>() for the preprocess described by `a`
+template <typename F>
+void with_pre_types(const PreArgs& a, F f) {
+  const bool dense = is_dense(a.so, a.H, a.L1, a.L2, a.D) && is_dense(a.sdo, a.H, a.L1, a.L2, a.D);
+  const bool resid = a.o_resid != nullptr;
+  auto by_layout = [&](auto d, auto bf) {
+    using T = std::true_type;
+    using N = std::false_type;
+    if (dense) resid ? f(d, bf, T{}, T{}) : f(d, bf, T{}, N{});
+    else resid ? f(d, bf, N{}, T{}) : f(d, bf, N{}, N{});
   };
   using I32 = std::integral_constant<int, 32>;
   using I64 = std::integral_constant<int, 64>;
-  if (D == 32) {
-    if (bf16) pick(I32{}, std::true_type{}); else pick(I32{}, std::false_type{});
-  } else {
-    if (bf16) pick(I64{}, std::true_type{}); else pick(I64{}, std::false_type{});
-  }
+  if (a.D == 32) a.bf16 ? by_layout(I32{}, std::true_type{}) : by_layout(I32{}, std::false_type{});
+  else a.bf16 ? by_layout(I64{}, std::true_type{}) : by_layout(I64{}, std::false_type{});
+}
+int pre_grid(const PreArgs& a) { return grid_for(static_cast<long long>(a.B) * a.H * a.L1 * a.L2 * (a.D / 8), 256); }
+}  // namespace
+
+int launch_preprocess(const PreArgs& a, cudaStream_t stream) {
+  with_pre_types(a, [&](auto d, auto bf, auto dense, auto resid) {
+    preprocess_kernel<decltype(d)::value, decltype(bf)::value, decltype(dense)::value, decltype(resid)::value>
+        <<<pre_grid(a), 256, 0, stream>>>(a);
+  });
   return static_cast<int>(cudaGetLastError());
 }
 
 int launch_mask_bias(const void* bias, const long long sb[4], const uint8_t* key_mask, void* out, int B, int H, int L2,
                      int L2p, bool bf16, cudaStream_t stream) {
   const int grid = grid_for(static_cast<long long>(B) * H * L2p * (L2p / 8), 256);
-  if (bf16)
-    mask_bias_kernel<true><<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(bias), sb[0], sb[1], sb[2], key_mask,
-                                                     static_cast<uint16_t*>(out), B * H, H, L2, L2p);
-  else
-    mask_bias_kernel<false><<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(bias), sb[0], sb[1], sb[2], key_mask,
-                                                      static_cast<uint16_t*>(out), B * H, H, L2, L2p);
+  const bool vec = L2 % 8 == 0 && sb[0] % 8 == 0 && sb[1] % 8 == 0 && sb[2] % 8 == 0 && sb[3] == 1 &&
+                   reinterpret_cast<uintptr_t>(bias) % 16 == 0 && reinterpret_cast<uintptr_t>(key_mask) % 8 == 0;
+  auto go = [&](auto kern) {
+    kern<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(bias), sb[0], sb[1], sb[2], sb[3], key_mask,
+                                   static_cast<uint16_t*>(out), B * H, H, L2, L2p);
+  };
+  if (vec) {
+    if (bf16) go(mask_bias_kernel<true, true>);
+    else go(mask_bias_kernel<false, true>);
+  } else {
+    if (bf16) go(mask_bias_kernel<true, false>);
+    else go(mask_bias_kernel<false, false>);
+  }
   return static_cast<int>(cudaGetLastError());
 }
 
 int launch_bwd_prologue(const void* bias, const long long sb[4], void* bias_t, int B, int H, int L2, float* dq32,
-                        long long dq_elems, cudaStream_t stream) {
+                        long long dq_elems, const PreArgs* pre, cudaStream_t stream) {
   const int sms = num_sms();
   const long long tiles = static_cast<long long>(L2 / 64) * (L2 / 64) * B * H;
   const int tr_blocks = static_cast<int>(tiles < 2LL * sms ? tiles : 2LL * sms);
-  const int grid = tr_blocks + 6 * sms;
-  bwd_prologue_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(bias), static_cast<uint16_t*>(bias_t),
-                                                B * H, H, L2, sb[0], sb[1], sb[2], tr_blocks,
-                                                reinterpret_cast<float4*>(dq32), dq_elems / 4);
+  const int zero_blocks = grid_for(dq_elems / 4, 256) < 6 * sms ? grid_for(dq_elems / 4, 256) : 6 * sms;
+  auto go = [&](auto kern, int pre_blocks, const PreArgs& a) {
+    kern<<<tr_blocks + zero_blocks + pre_blocks, 256, 0, stream>>>(
+        static_cast<const uint16_t*>(bias), static_cast<uint16_t*>(bias_t), B * H, H, L2, sb[0], sb[1], sb[2], tr_blocks,
+        reinterpret_cast<float4*>(dq32), dq_elems / 4, pre_blocks, a);
+  };
+  if (pre)
+    with_pre_types(*pre, [&](auto d, auto bf, auto dense, auto resid) {
+      go(bwd_prologue_kernel<true, decltype(d)::value, decltype(bf)::value, decltype(dense)::value, decltype(resid)::value>,
+         pre_grid(*pre), *pre);
+    });
+  else
+    go(bwd_prologue_kernel<false, 32, true, true, true>, 0, PreArgs{});
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -640,7 +652,7 @@ int launch_bwd_epilogue(const float* dq32, void* dq, const long long sdq[4], int
                         Status status, cudaStream_t stream) {
   const long long rows = static_cast<long long>(B) * H * L1 * L2;
   const int dq_blocks = grid_for(rows * (D / 8), 256);
-  const int db_blocks = ((L2 + 63) / 64) * ((L2 + 63) / 64) * B * H;
+  const int db_blocks = ((L2 + 31) / 32) * ((L2 + 31) / 32) * B * H;
   const int grid = dq_blocks + db_blocks;
   uint16_t* out = static_cast<uint16_t*>(dq);
   uint16_t* cast = static_cast<uint16_t*>(dbias_cast);

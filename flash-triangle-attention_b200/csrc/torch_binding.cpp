@@ -149,7 +149,6 @@ ForwardOut run_forward(const at::Tensor& q_, const at::Tensor& k_, const at::Ten
   r.q = dense(q_);
   r.k = dense(k_);
   r.v = dense(v_);
-  r.bias = dense(bias_);
   const FtaProblem prob = problem_of(q_);
   const int64_t l2p = padded(prob.L2);
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
@@ -158,15 +157,15 @@ ForwardOut run_forward(const at::Tensor& q_, const at::Tensor& k_, const at::Ten
     // Ragged L2 and / or a boolean key mask: only this bias-sized tensor is staged (whole 128-blocks,
     // -inf on padding and masked keys); q, k, v are read in place.
     at::Tensor km;
-    if (key_mask.has_value()) {
-      km = key_mask->to(q_.device()).contiguous();
-      if (reinterpret_cast<uintptr_t>(km.data_ptr()) % 8 != 0) km = km.clone();
-    }
-    at::Tensor staged = at::empty({prob.B, prob.H, l2p, l2p}, q_.options());
-    const FtaTensor4 b4 = v4(r.bias);
-    check_rc(fta_mask_bias(&prob, &b4, km.defined() ? static_cast<const uint8_t*>(km.data_ptr()) : nullptr,
-                           staged.data_ptr(), stream), "fta_mask_bias");
-    r.bias = staged;
+    if (key_mask.has_value()) km = key_mask->to(q_.device()).contiguous();
+    r.bias = at::empty({prob.B, prob.H, l2p, l2p}, q_.options());
+    FtaTensor4 b4;
+    b4.ptr = bias_.data_ptr();
+    for (int i = 0; i < 4; ++i) b4.stride[i] = bias_.stride(i);
+    check_rc(fta::native_mask_bias(prob, b4, km.defined() ? static_cast<const uint8_t*>(km.data_ptr()) : nullptr,
+                                   r.bias.data_ptr(), stream), "fta_mask_bias");
+  } else {
+    r.bias = dense(bias_);
   }
   float* lse = nullptr;
   void* resid = nullptr;
@@ -253,7 +252,6 @@ void check_arguments(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
   const int64_t l2 = q.size(3);
   require(bias.sizes() == at::IntArrayRef({q.size(0), q.size(1), l2, l2}), "bias must be (B, H, L2, L2)");
   require(k.device() == q.device() && v.device() == q.device() && bias.device() == q.device(), "q, k, v and the bias must be on one device");
-  require(l2 % 8 == 0, "the kernels address rows of L2 elements with 16-byte steps (attention() pads other L2)");
   if (key_mask.has_value())
     require(key_mask->scalar_type() == at::kBool && key_mask->sizes() == at::IntArrayRef({q.size(0), l2}), "key_mask: bool (B, L2)");
   ensure_status(q.device());

@@ -158,15 +158,15 @@ def attention(q, k, v, b_pw, sm_scale, group=None, key_mask=None):
     True = attend) removes keys, and ``L2`` need not be a multiple of 128. Both are handled inside
     the kernels - ragged last blocks are padded by the tile loads and clipped by the stores, masked
     keys get exactly zero probability and exactly zero dBias, dK, dV - and only a bias-sized tensor
-    is staged; q, k, v are never copied. (An ``L2`` that is not a multiple of 8 is first padded to
-    one: the kernels step through rows of ``L2`` elements 16 bytes at a time.) A query whose every
-    key is masked gets a zero output row and zero gradients."""
+    is staged; q, k, v are never copied. (With a ``group``, an ``L2`` that is not a multiple of 8 is first
+    padded to one: the sum over the group rounds rows of ``L2`` elements 16 bytes at a time.) A query whose
+    every key is masked gets a zero output row and zero gradients."""
     B, H, L1, L2, D = q.shape
     if key_mask is not None:
         if key_mask.dim() == 4:
             key_mask = key_mask.reshape(key_mask.shape[0], L2)
         key_mask = key_mask.expand(B, L2)
-    if L2 % 8 == 0:
+    if group is None or L2 % 8 == 0:
         return _call(q, k, v, b_pw, sm_scale, group, key_mask)
     pad = (L2 + 7) // 8 * 8 - L2
     F = torch.nn.functional  # F.pad is differentiable: gradients of the padding are dropped on the way back

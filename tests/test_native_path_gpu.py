@@ -1,8 +1,11 @@
-"""The native call path of ``attention()`` where it branches: with and without a backward pass to come."""
+"""The native call path of ``attention()`` where it branches: with and without a backward pass to come, any L2,
+small and unequal shares of rows."""
+import numpy as np
 import pytest
 import torch
 
 import flash_tt_attn as fta
+from oracle import tt_attn_oracle as npo
 
 pytestmark = pytest.mark.gpu
 
@@ -21,3 +24,64 @@ def test_forward_without_a_backward_pass_gives_the_same_output(L1, L2, D, dtype)
     fta.check_device_status()
     assert plain.grad_fn is None and quiet.grad_fn is None and kept.grad_fn is not None
     assert torch.equal(plain, kept) and torch.equal(plain, quiet)
+
+
+@pytest.mark.parametrize("B,H,L1,L2,D,dtype,masked", [
+    (1, 1, 1, 1, 32, "fp16", False), (2, 1, 3, 7, 32, "bf16", True), (1, 2, 4, 33, 64, "fp16", False),
+    (1, 2, 7, 127, 32, "bf16", True), (2, 1, 5, 129, 32, "fp16", True), (1, 1, 9, 317, 64, "bf16", False),
+    (1, 1, 67, 261, 32, "bf16", True), (1, 1, 150, 130, 64, "fp16", False), (1, 3, 70, 12, 32, "bf16", False),
+])
+def test_any_l2_with_and_without_a_mask(B, H, L1, L2, D, dtype, masked):
+    """L2 of any size: rows of the bias and of dBias that start at any alignment, padded planes, last blocks of
+    every length; up to 64 dBias planes, row groups that do not come out even."""
+    dt = {"fp16": torch.float16, "bf16": torch.bfloat16}[dtype]
+    g = torch.Generator().manual_seed(L1 * 1000 + L2)
+    q, k, v, do = (torch.randn(B, H, L1, L2, D, generator=g).to(dt) for _ in range(4))
+    bias = torch.randn(B, H, L2, L2, generator=g).to(dt)
+    mask = None
+    if masked:
+        mask = torch.rand(B, L2, generator=g) > 0.2
+        mask[:, 0] = True
+    leaves = [a.cuda().requires_grad_(True) for a in (q, k, v, bias)]
+    o = fta.attention(*leaves, D ** -0.5, key_mask=None if mask is None else mask.cuda())
+    o.backward(do.cuda())
+    fta.check_device_status()
+    bm = bias.float()
+    if mask is not None:
+        bm = torch.where(mask[:, None, None, :], bm, torch.tensor(-1.0e9))
+    ref = npo.forward_backward(q.float().numpy(), k.float().numpy(), v.float().numpy(), bm.numpy(), do.float().numpy(), D ** -0.5)
+    got = {"o": o, "dq": leaves[0].grad, "dk": leaves[1].grad, "dv": leaves[2].grad, "dbias": fta.last_dbias_f32()}
+    assert leaves[3].grad.shape == bias.shape and got["dbias"].shape == bias.shape
+    for name, t in got.items():
+        a = t.detach().float().cpu().numpy()
+        assert np.isfinite(a).all(), name
+        assert npo.max_abs(a, ref[name]) <= 2e-2, (name, npo.max_abs(a, ref[name]))
+        if np.linalg.norm(ref[name]) > 1e-6:
+            assert npo.rel_l2(a, ref[name]) <= 1e-2, (name, npo.rel_l2(a, ref[name]))
+    want = got["dbias"].to(dt)
+    assert torch.equal(leaves[3].grad, want)
+
+
+@pytest.mark.parametrize("D,L1,L2", [(64, 6, 512), (64, 40, 256), (32, 7, 640)])
+def test_backward_is_bit_reproducible_over_many_blocks(D, L1, L2):
+    """Many flushes of the dBias boxes through few spare buffers: a box sent twice or too early shows as a
+    difference between runs, or from the sum over two shares of the rows."""
+    g = torch.Generator(device="cuda").manual_seed(D + L2)
+    q, k, v, do = (torch.randn(1, 4, L1, L2, D, device="cuda", dtype=torch.bfloat16, generator=g) for _ in range(4))
+    b = torch.randn(1, 4, L2, L2, device="cuda", dtype=torch.bfloat16, generator=g)
+
+    def run(rows):
+        t = [x[:, :, rows].contiguous().requires_grad_() for x in (q, k, v)]
+        bb = b.clone().requires_grad_()
+        o = fta.attention(*t, bb, 0.2)
+        o.backward(do[:, :, rows].contiguous())
+        return [o.detach(), t[1].grad, t[2].grad, fta.last_dbias_f32()]
+
+    first = run(slice(0, L1))
+    for _ in range(3):
+        assert all(torch.equal(x, y) for x, y in zip(first, run(slice(0, L1))))
+    parts = [run(slice(0, L1 // 2)), run(slice(L1 // 2, L1))]
+    for i in range(3):
+        assert torch.equal(torch.cat([p[i] for p in parts], dim=2), first[i])
+    assert torch.allclose(parts[0][3] + parts[1][3], first[3], atol=1e-4, rtol=1e-5)
+    fta.check_device_status()
