@@ -543,6 +543,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     bool ok = true;
     int tt = 0, nb = 0, slot = 0;
     uint32_t ring_par = 0;
+    uint32_t q_in = 0, b_in = 0;  // early polls: statistics of the next tile, bias of the next query block
     for (int n = 0; n < ngroups && ok; ++n) {
       const int Gc = min(G, row_end - (row_begin + n * G));
       for (int jb = 0; jb < nq && ok; ++jb, ++nb) {
@@ -550,11 +551,11 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
         for (int c = 0; c < 32; ++c) acc[c] = mk2(0.f, 0.f);
         const int bs = 2 * (nb & 1) + hf;
-        ok = mbar_wait_warp(bar(C::B_BIASFULL + bs), (nb >> 1) & 1, w, 0x41);
+        ok = mbar_finish_wait(b_in, bar(C::B_BIASFULL + bs), (nb >> 1) & 1, w, 0x41);
         if (!ok) break;
 #pragma unroll 1
         for (int g = 0; g < Gc; ++g, ++tt) {
-          ok = mbar_wait_warp(bar(C::B_QDOFULL + 2 * slot + hf), ring_par, w, 0x43) &&  // statistics visible
+          ok = mbar_finish_wait(q_in, bar(C::B_QDOFULL + 2 * slot + hf), ring_par, w, 0x43) &&  // statistics visible
                mbar_wait_warp(bar(C::B_XFULL + hf), tt & 1, w, 0x42);
           if (!ok) break;
           tc_fence_after_sync();
@@ -658,6 +659,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             st_shared_v4(my_ds + ((j ^ (key & 7)) << 4), dd[4 * j], dd[4 * j + 1], dd[4 * j + 2], dd[4 * j + 3]);
+          q_in = mbar_test_wait(bar(C::B_QDOFULL + 2 * slot + hf), ring_par);
           tmem_st_wait();
           fence_proxy_async_smem();
           tc_fence_before_sync();
@@ -669,6 +671,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         // half bias stage (this thread's row of it, whose bias values nobody else reads), one in the spare box,
         // whose previous contents left while the block was worked on. With one spare box for both halves those are
         // the other half's; a barrier per half, each waited for once per block, never runs a phase ahead.
+        b_in = mbar_test_wait(bar(C::B_BIASFULL + (bs ^ 2)), ((nb + 1) >> 1) & 1);
         const int by = C::NX == 2 ? hf : hf ^ 1;                         // who parked there last
         const int use = (C::NX == 2 || hf == 0) ? nb - 1 : nb;           // in which block
         if (use >= 0) {

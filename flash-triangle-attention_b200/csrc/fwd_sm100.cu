@@ -290,6 +290,7 @@ fta_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const f32x2 scale2 = mk2(p.scale, p.scale);
     const f32x2 log2e2 = mk2(kLog2e, kLog2e);
     int n = 0, nbias = 0;
+    uint32_t s_in = 0;
     bool ok = true;
     for (int u = 0; u < nunits && ok; ++u) {
     const int i0 = unit_i0(u);
@@ -305,12 +306,12 @@ fta_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       const uint8_t* brow = sBias + bs * C::BIAS_B + row * 128;
       for (int gi = 0; gi < ngi; ++gi, ++n) {
         const int g = 2 * gi + wg;
-        ok = mbar_wait_warp(bar(C::B_SFULL + wg), n & 1, w, 6);
+        uint32_t bias_in = 1;
+        if (gi == 0) bias_in = mbar_test_wait(bar(C::B_BIASFULL + bs), (nbias >> 1) & 1);
+        ok = mbar_finish_wait(s_in, bar(C::B_SFULL + wg), n & 1, w, 6);
         if (!ok) break;
-        if (gi == 0) {
-          ok = mbar_wait_warp(bar(C::B_BIASFULL + bs), (nbias >> 1) & 1, w, 7);
-          if (!ok) break;
-        }
+        ok = mbar_finish_wait(bias_in, bar(C::B_BIASFULL + bs), (nbias >> 1) & 1, w, 7);
+        if (!ok) break;
         tc_fence_after_sync();
         uint32_t sr[128];
 #pragma unroll
@@ -320,6 +321,9 @@ fta_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(C::B_SFREE + wg));
+        // the P buffer is free once the PV MMA of this warpgroup's previous tile is done
+        uint32_t p_free = 1;
+        if (n > 0) p_free = mbar_test_wait(bar(C::B_PVDONE + wg), (n - 1) & 1);
         // pass 1: x = s*scale + bias (natural-log units), row max
         float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
@@ -378,9 +382,8 @@ fta_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             tmem_st32(ta, orr);
           }
         }
-        // the P buffer is free once the PV MMA of this warpgroup's previous tile is done
         if (n > 0) {
-          ok = mbar_wait_warp(bar(C::B_PVDONE + wg), (n - 1) & 1, w, 10);
+          ok = mbar_finish_wait(p_free, bar(C::B_PVDONE + wg), (n - 1) & 1, w, 10);
           if (!ok) break;
         }
         // pass 2: p = 2^((x - m) * log2e), row sum, pack, hand P to the tensor core through TMEM
@@ -429,6 +432,7 @@ fta_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         }
         float s0, s1;
         un2(add2(sum2a, sum2b), s0, s1);
+        s_in = mbar_test_wait(bar(C::B_SFULL + wg), (n + 1) & 1);  // of the next tile
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
