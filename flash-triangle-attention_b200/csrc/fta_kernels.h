@@ -35,6 +35,23 @@ inline cudaError_t ensure_dynamic_smem(PerDeviceOnce& once, Kernel kern, int byt
   return e;
 }
 
+// Launches `kern` so that it may start while the kernel before it on the stream still runs (programmatic stream
+// serialization); `kern` calls grid_dependency_wait() before it touches memory.
+template <typename Kernel, typename... Args>
+inline cudaError_t launch_overlapped(Kernel kern, dim3 grid, int threads, int smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // SM count of the current device, looked up once per device (the attribute call costs more than the
 // rest of a launch's host arithmetic).
 inline int num_sms() {

@@ -365,6 +365,7 @@ template <bool kBf16, bool kVec>
 __global__ void __launch_bounds__(256) mask_bias_kernel(const uint16_t* __restrict__ bias, long long s_b, long long s_h,
                                                         long long s_q, long long s_k, const uint8_t* __restrict__ key_mask,
                                                         uint16_t* __restrict__ out, int BH, int H, int L2, int L2p) {
+  grid_launch_dependents();
   constexpr uint32_t NEG_INF = kBf16 ? 0xFF80u : 0xFC00u;
   const int vec_per_row = L2p / 8;
   const long long total = static_cast<long long>(BH) * L2p * vec_per_row;

@@ -171,6 +171,11 @@ __device__ __forceinline__ bool mbar_finish_wait(uint32_t early, uint32_t bar, u
   return mbar_wait_warp(bar, parity, w, site);
 }
 
+// Programmatic dependent launch: wait until the kernel before is complete and its writes are visible / let the next
+// kernel on the stream be launched (its blocks start as this grid's leave room).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Host-visible copy of a status word (see Status in fta_kernels.h): one thread, nothing to do while the
 // word is zero.
 __device__ __forceinline__ void publish_status(const int* word, int* mirror) {
