@@ -97,7 +97,9 @@ struct BwdArgs {
   CUtensorMap tmPlane; // the partial dBias planes as (nplanes*B*H, L2 keys, L2 queries) float32, same box
   const float* lse;    // (3,B,H,L1,L2): -max, -log2(sum), combined (NaN where inexact)
   const float* delta;  // (B,H,L1,L2)
-  float* dq32;         // (B,H,L1,L2,D) float32, zeroed; receives sum over key blocks of dS K
+  float* dq32;         // (B,H,L1,L2,D) float32: dq_parts == 0: one, zeroed, receives the sum over key blocks of dS K;
+                       // else one per key block
+  int dq_parts;
   void* dk;
   void* dv;
   int* status;
@@ -137,10 +139,10 @@ int launch_mask_bias(const void* bias, const long long sb[4], const uint8_t* key
 int launch_bwd_prologue(const void* bias, const long long sb[4], void* bias_t, int B, int H, int L2, float* dq32,
                         long long dq_elems, const PreArgs* pre, cudaStream_t stream);
 
-// Backward epilogue, one launch: dq[row, d] = (dtype)(scale * dq32[row, d]) and, for the KEY-MAJOR
+// Backward epilogue, one launch: dq[row, d] = (dtype)(scale * sum of the `dq_parts` dq32[part][row, d]) and, for the KEY-MAJOR
 // planes the backward kernel writes, (nplanes, B*H, key, query) with rows of L2 rounded up to 8 elements:
 // dbias_f32[bh][query][key] = sum_p planes[p][bh][key][query] in plane order, optional rounded copy
-int launch_bwd_epilogue(const float* dq32, void* dq, const long long sdq[4], int B, int H, int L1, int L2, int D,
+int launch_bwd_epilogue(const float* dq32, int dq_parts, void* dq, const long long sdq[4], int B, int H, int L1, int L2, int D,
                         float scale, const float* planes, int nplanes, float* dbias_f32, void* dbias_cast, bool bf16,
                         Status status, cudaStream_t stream);
 
