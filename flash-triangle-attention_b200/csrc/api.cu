@@ -88,18 +88,10 @@ size_t dq32_bytes(const FtaProblem* p) {
   return static_cast<size_t>(p->B) * p->H * p->L1 * p->L2 * p->D * sizeof(float);
 }
 // float32 dQ accumulator, dBias planes, key-major copy of the bias (16-bit, whole blocks)
-size_t workspace_bytes(const FtaProblem* p, int nplanes, int dq_parts) {
+size_t workspace_bytes(const FtaProblem* p, int nplanes) {
   const size_t l2p = static_cast<size_t>(padded_l2(p));
-  return align256(dq32_bytes(p) * (dq_parts > 1 ? dq_parts : 1)) + align256(plane_bytes(p) * nplanes) +
+  return align256(dq32_bytes(p)) + align256(plane_bytes(p) * nplanes) +
          align256(static_cast<size_t>(p->B) * p->H * l2p * l2p * 2);
-}
-// How dQ is summed over the key blocks: each block stores a float32 part of its own (1 or 2 parts), or all are added
-// into one zeroed buffer (0). Two parts cost the finalise kernel a second read, as much as the zero fill that they save,
-// and the main kernel's stores leave an SM at 30 bytes per cycle instead of 24; more parts would cost more than that.
-// Where the workspace is bounded (the C ABI: fixed arrays, documented sizes) only the part that costs nothing.
-int plan_dq_parts(const FtaProblem* p, bool bounded) {
-  const int key_blocks = padded_l2(p) / 128;
-  return key_blocks == 1 ? 1 : key_blocks == 2 && !bounded ? 2 : 0;
 }
 int plan_planes(const FtaProblem* p) { return fta::bwd_num_planes(p->B, p->H, p->L1, p->L2, p->D, fta::num_sms()); }
 
@@ -157,7 +149,7 @@ int fill_pre(fta::PreArgs* a, const FtaProblem* prob, const FtaTensor5* o, const
 }
 
 // `pre`: also run the preprocess it describes, in the launch of the prologue (nullptr: delta is there already)
-int backward(const FtaProblem* prob, int nplanes, int dq_parts, const fta::PreArgs* pre, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
+int backward(const FtaProblem* prob, int nplanes, const fta::PreArgs* pre, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
              const FtaTensor4* bias, const FtaTensor5* dout, const float* lse, const float* delta, float sm_scale,
              const FtaTensor5* dq, const FtaTensor5* dk, const FtaTensor5* dv, float* dbias_f32, void* dbias_cast,
              void* workspace, size_t have_bytes, fta::Status status, cudaStream_t st) {
@@ -169,13 +161,14 @@ int backward(const FtaProblem* prob, int nplanes, int dq_parts, const fta::PreAr
   // the kernel fetches the statistics with 512-byte bulk copies and the epilogue writes dBias with
   // 16-byte stores
   if (!aligned16(lse) || !aligned16(delta) || !aligned16(dbias_f32) || !aligned16(dbias_cast)) return FTA_ERR_ALIGN;
-  if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0 || have_bytes < workspace_bytes(prob, nplanes, dq_parts))
+  if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0 || have_bytes < workspace_bytes(prob, nplanes))
     return FTA_ERR_WORKSPACE;
   const size_t rows = static_cast<size_t>(prob->B) * prob->H * prob->L1 * prob->L2;
   float* dq32 = static_cast<float*>(workspace);
-  float* planes = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(dq32_bytes(prob) * (dq_parts > 1 ? dq_parts : 1)));
+  float* planes = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(dq32_bytes(prob)));
   void* bias_t = reinterpret_cast<uint8_t*>(planes) + align256(plane_bytes(prob) * nplanes);
   const bool bf16 = prob->dtype == FTA_BF16;
+  const bool one_block = prob->L2 <= 128;  // one key block: the kernel writes dq itself
 
   fta::BwdArgs a;
   FtaTensor4 bt;  // key-major copy: (B, H, key, query) contiguous
@@ -192,7 +185,7 @@ int backward(const FtaProblem* prob, int nplanes, int dq_parts, const fta::PreAr
   {
     // dq32 seen as (B*H*L1, L2, D) float32; the kernel adds 32-query x 16-column tiles into it with
     // TMA reductions (the part of a ragged last query block beyond L2 is clipped)
-    const uint64_t bhi = static_cast<uint64_t>(prob->B) * prob->H * prob->L1 * (dq_parts > 1 ? dq_parts : 1);
+    const uint64_t bhi = static_cast<uint64_t>(prob->B) * prob->H * prob->L1;
     if (bhi >= (1ull << 31)) return FTA_ERR_SHAPE;  // tile coordinates are signed 32-bit
     const uint64_t dims[3] = {static_cast<uint64_t>(prob->D), static_cast<uint64_t>(prob->L2), bhi};
     const uint64_t str[3] = {0, static_cast<uint64_t>(prob->D) * 4, static_cast<uint64_t>(prob->L2) * prob->D * 4};
@@ -208,11 +201,11 @@ int backward(const FtaProblem* prob, int nplanes, int dq_parts, const fta::PreAr
   a.lse = lse;
   a.delta = delta;
   a.dq32 = dq32;
+  a.dq = dq->ptr;
   a.dk = dk->ptr;
   a.dv = dv->ptr;
   a.status = status.word;
   a.nplanes = nplanes;
-  a.dq_parts = dq_parts;
   a.B = prob->B;
   a.H = prob->H;
   a.L1 = prob->L1;
@@ -221,6 +214,7 @@ int backward(const FtaProblem* prob, int nplanes, int dq_parts, const fta::PreAr
   a.bf16 = bf16;
   long long sdq[4];
   for (int i = 0; i < 4; ++i) {
+    a.sdq[i] = dq->stride[i];
     a.sdk[i] = dk->stride[i];
     a.sdv[i] = dv->stride[i];
     sdq[i] = dq->stride[i];
@@ -230,12 +224,12 @@ int backward(const FtaProblem* prob, int nplanes, int dq_parts, const fta::PreAr
   long long sb[4];
   for (int i = 0; i < 4; ++i) sb[i] = bias->stride[i];
   if (const int e = fta::launch_bwd_prologue(bias->ptr, sb, bias_t, prob->B, prob->H, l2p, dq32,
-                                             dq_parts ? 0 : static_cast<long long>(rows) * prob->D, pre, st))
+                                             one_block ? 0 : static_cast<long long>(rows) * prob->D, pre, st))
     return cuda_fail(e);
   if (g_prof_start) cudaEventRecord(g_prof_start, st);
   if (const int e = fta::launch_bwd(a, st)) return cuda_fail(e);
   if (g_prof_stop) cudaEventRecord(g_prof_stop, st);
-  if (const int e = fta::launch_bwd_epilogue(dq32, dq_parts, dq->ptr, sdq, prob->B, prob->H, prob->L1, prob->L2, prob->D,
+  if (const int e = fta::launch_bwd_epilogue(one_block ? nullptr : dq32, dq->ptr, sdq, prob->B, prob->H, prob->L1, prob->L2, prob->D,
                                              sm_scale, planes, nplanes, dbias_f32, dbias_cast, bf16, status, st))
     return cuda_fail(e);
   return FTA_OK;
@@ -269,8 +263,7 @@ int native_mask_bias(const FtaProblem& prob, const FtaTensor4& bias, const uint8
 int native_backward_plan(const FtaProblem& prob, BackwardPlan* plan) {
   if (const int rc = check_problem(&prob, true)) return rc;
   plan->nplanes = plan_planes(&prob);
-  plan->dq_parts = plan_dq_parts(&prob, false);
-  plan->workspace_bytes = workspace_bytes(&prob, plan->nplanes, plan->dq_parts);
+  plan->workspace_bytes = workspace_bytes(&prob, plan->nplanes);
   plan->delta_bytes = sizeof(float) * static_cast<size_t>(prob.B) * prob.H * prob.L1 * padded_l2(&prob);
   return FTA_OK;
 }
@@ -283,7 +276,7 @@ int native_backward(const FtaProblem& prob, const BackwardPlan& plan, const FtaT
   float* delta = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + plan.workspace_bytes);
   fta::PreArgs pre;
   if (const int rc = fill_pre(&pre, &prob, &o, o_resid, &dout, delta)) return rc;
-  return backward(&prob, plan.nplanes, plan.dq_parts, &pre, &q, &k, &v, &bias, &dout, lse, delta, sm_scale, &dq, &dk, &dv, dbias_f32,
+  return backward(&prob, plan.nplanes, &pre, &q, &k, &v, &bias, &dout, lse, delta, sm_scale, &dq, &dk, &dv, dbias_f32,
                   dbias_cast, workspace, plan.workspace_bytes, {status.word, status.mirror}, stream);
 }
 
@@ -347,7 +340,7 @@ int fta_mask_bias(const FtaProblem* prob, const FtaTensor4* bias, const uint8_t*
 int fta_bwd_num_planes(const FtaProblem* prob) { return check_problem(prob) ? 0 : plan_planes(prob); }
 
 size_t fta_bwd_workspace_bytes(const FtaProblem* prob) {
-  return check_problem(prob) ? 0 : workspace_bytes(prob, plan_planes(prob), plan_dq_parts(prob, true));
+  return check_problem(prob) ? 0 : workspace_bytes(prob, plan_planes(prob));
 }
 
 int fta_backward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* k, const FtaTensor5* v,
@@ -356,7 +349,7 @@ int fta_backward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* 
                  float* dbias_f32, void* dbias_cast, void* workspace, size_t workspace_bytes, int32_t* status,
                  void* stream) {
   if (const int rc = check_problem(prob)) return rc;
-  return backward(prob, plan_planes(prob), plan_dq_parts(prob, true), nullptr, q, k, v, bias, dout, lse, delta, sm_scale, dq, dk, dv, dbias_f32, dbias_cast,
+  return backward(prob, plan_planes(prob), nullptr, q, k, v, bias, dout, lse, delta, sm_scale, dq, dk, dv, dbias_f32, dbias_cast,
                   workspace, workspace_bytes, {status, nullptr}, static_cast<cudaStream_t>(stream));
 }
 

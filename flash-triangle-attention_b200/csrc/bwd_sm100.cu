@@ -30,8 +30,8 @@
 // only ever touched by one CTA, one addition per group, each completed before the next, so the result is
 // bit-exact run to run; the planes are summed in fixed order by the finalise kernel.
 // dQ leaves the CTA the same way: TMEM -> shared memory -> TMA reduction into a zero-initialised
-// float32 buffer (sum over key blocks), or, with one or two key blocks, a TMA store into a part of its own per key
-// block, which needs no zeros and leaves the SM a quarter faster; the finalise kernel adds the parts. Whatever the route (TMA or register stores, tiles or contiguous), an SM
+// float32 buffer (sum over key blocks). With a single key block (L2 <= 128) there is nothing to add up: dQ is scaled,
+// rounded and stored like dK and dV, and neither zero fill nor finalisation is needed. Whatever the route (TMA or register stores, tiles or contiguous), an SM
 // gets out 32 bytes per cycle of stores and 25 of float32 reductions (30 and 24 with all SMs at it): at D = 32 a tile's
 // 16 KB of dQ and third of 64 KB of dBias need 1 560 cycles, at D = 64 32 KB and 64 KB need 4 100.
 //
@@ -110,15 +110,15 @@ struct BwdParams {
   const float* lse;  // three planes: -max (natural-log units), -log2(sum), c (see the forward kernel)
   const float* delta;
   float* dq32;
+  void* dq;  // written by the kernel itself where L2 <= 128
   void* dk;
   void* dv;
   int* status;
   int H, L1, L2, NP, BH;
   int stat_pitch;  // row pitch of lse / delta: L2 rounded up to 128
-  long long sdk[4], sdv[4];
+  long long sdq[4], sdk[4], sdv[4];
   float scale;  // sm_scale
   long long stat_stride;  // elements between the statistics planes
-  int dq_part_rows;  // 0: dQ tiles are added up; else stored, B*H*L1 rows (of L2 x D) per key block
 };
 
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -463,6 +463,18 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t stage = smem_u32(sDQ) + (warp & 3) * 2048;
     const bool key_live = kb * 128 + lrow < p.L2;  // keys past L2 in a ragged block own no output row
+    // 16 columns of this thread's row, scaled and rounded
+    auto store16 = [&](uint16_t* out, const uint32_t (&x)[16], float mul) {
+#pragma unroll
+      for (int v4 = 0; v4 < 2; ++v4) {
+        uint4 ov;
+        ov.x = pack2<kBf16>(__uint_as_float(x[v4 * 8 + 0]) * mul, __uint_as_float(x[v4 * 8 + 1]) * mul);
+        ov.y = pack2<kBf16>(__uint_as_float(x[v4 * 8 + 2]) * mul, __uint_as_float(x[v4 * 8 + 3]) * mul);
+        ov.z = pack2<kBf16>(__uint_as_float(x[v4 * 8 + 4]) * mul, __uint_as_float(x[v4 * 8 + 5]) * mul);
+        ov.w = pack2<kBf16>(__uint_as_float(x[v4 * 8 + 6]) * mul, __uint_as_float(x[v4 * 8 + 7]) * mul);
+        if (key_live) *reinterpret_cast<uint4*>(out + v4 * 8) = ov;
+      }
+    };
     bool ok = true;
     int tt = 0;
     for (int n = 0; n < ngroups && ok; ++n) {
@@ -483,6 +495,11 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             if (c == kD / 16 - 1) tc_fence_before_sync();
             __syncwarp();
             if (c == kD / 16 - 1 && lane == 0) mbar_arrive(bar(C::B_DQFREE + buf));
+            if (nkb == 1) {
+              store16(reinterpret_cast<uint16_t*>(p.dq) + b * p.sdq[0] + h * p.sdq[1] + static_cast<long long>(i0 + g) * p.sdq[2] +
+                          static_cast<long long>(lrow) * p.sdq[3] + c * 16, qv, p.scale);
+              continue;
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j)  // 64-byte swizzle
               st_shared_v4(stage + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4), qv[4 * j], qv[4 * j + 1], qv[4 * j + 2],
@@ -490,9 +507,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             fence_proxy_async_smem();
             __syncwarp();
             if (elect_one()) {
-              const int drow = bh * p.L1 + i0 + g;
-              if (p.dq_part_rows) tma_store_3d(&tmDQ, stage, c * 16, jb * 128 + (warp & 3) * 32, kb * p.dq_part_rows + drow);
-              else tma_reduce_add_3d(&tmDQ, stage, c * 16, jb * 128 + (warp & 3) * 32, drow);
+              tma_reduce_add_3d(&tmDQ, stage, c * 16, jb * 128 + (warp & 3) * 32, bh * p.L1 + i0 + g);
               bulk_commit_group();
             }
             __syncwarp();
@@ -517,15 +532,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(C::B_ACCFREE + g));
               }
-#pragma unroll
-              for (int v4 = 0; v4 < 2; ++v4) {
-                uint4 ov;
-                ov.x = pack2<kBf16>(__uint_as_float(av[v4 * 8 + 0]) * mul, __uint_as_float(av[v4 * 8 + 1]) * mul);
-                ov.y = pack2<kBf16>(__uint_as_float(av[v4 * 8 + 2]) * mul, __uint_as_float(av[v4 * 8 + 3]) * mul);
-                ov.z = pack2<kBf16>(__uint_as_float(av[v4 * 8 + 4]) * mul, __uint_as_float(av[v4 * 8 + 5]) * mul);
-                ov.w = pack2<kBf16>(__uint_as_float(av[v4 * 8 + 6]) * mul, __uint_as_float(av[v4 * 8 + 7]) * mul);
-                if (key_live) *reinterpret_cast<uint4*>(optr + v4 * 8) = ov;
-              }
+              store16(optr, av, mul);
             }
           }
         }
@@ -724,6 +731,7 @@ int launch_bwd_t(const BwdArgs& a, int NP, cudaStream_t stream) {
   p.lse = a.lse;
   p.delta = a.delta;
   p.dq32 = a.dq32;
+  p.dq = a.dq;
   p.dk = a.dk;
   p.dv = a.dv;
   p.status = a.status;
@@ -733,11 +741,11 @@ int launch_bwd_t(const BwdArgs& a, int NP, cudaStream_t stream) {
   p.NP = NP;
   p.BH = a.B * a.H;
   for (int i = 0; i < 4; ++i) {
+    p.sdq[i] = a.sdq[i];
     p.sdk[i] = a.sdk[i];
     p.sdv[i] = a.sdv[i];
   }
   p.scale = a.sm_scale;
-  p.dq_part_rows = a.dq_parts ? a.B * a.H * a.L1 : 0;
   p.stat_pitch = (a.L2 + 127) / 128 * 128;
   p.stat_stride = static_cast<long long>(a.B) * a.H * a.L1 * p.stat_pitch;
   const int grid = a.B * a.H * NP * ((a.L2 + 127) / 128);

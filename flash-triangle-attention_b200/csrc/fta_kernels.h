@@ -97,16 +97,15 @@ struct BwdArgs {
   CUtensorMap tmPlane; // the partial dBias planes as (nplanes*B*H, L2 keys, L2 queries) float32, same box
   const float* lse;    // (3,B,H,L1,L2): -max, -log2(sum), combined (NaN where inexact)
   const float* delta;  // (B,H,L1,L2)
-  float* dq32;         // (B,H,L1,L2,D) float32: dq_parts == 0: one, zeroed, receives the sum over key blocks of dS K;
-                       // else one per key block
-  int dq_parts;
+  float* dq32;         // (B,H,L1,L2,D) float32, zeroed; receives sum over key blocks of dS K (not used for L2 <= 128)
+  void* dq;            // written where L2 <= 128
   void* dk;
   void* dv;
   int* status;
   int B, H, L1, L2, D;
   int nplanes;  // bwd_num_planes()
   bool bf16;
-  long long sdk[4], sdv[4];  // element strides of dK, dV over (B, H, L1, L2)
+  long long sdq[4], sdk[4], sdv[4];  // element strides of dQ, dK, dV over (B, H, L1, L2)
   float sm_scale;
 };
 int launch_bwd(const BwdArgs& a, cudaStream_t stream);
@@ -134,15 +133,15 @@ int launch_mask_bias(const void* bias, const long long sb[4], const uint8_t* key
                      int L2p, bool bf16, cudaStream_t stream);
 
 // Backward prologue, one launch: bias_t[bh][k][q] = bias[b][h][q][k] (16-bit elements; `sb` = element
-// strides of the bias) and zero-fill of the float32 dQ accumulator (`dq_elems` floats, a multiple of 4); with `pre`
+// strides of the bias) and zero-fill of the float32 dQ accumulator (`dq_elems` floats, a multiple of 4, or 0); with `pre`
 // the preprocess too (three independent streams that share the launch)
 int launch_bwd_prologue(const void* bias, const long long sb[4], void* bias_t, int B, int H, int L2, float* dq32,
                         long long dq_elems, const PreArgs* pre, cudaStream_t stream);
 
-// Backward epilogue, one launch: dq[row, d] = (dtype)(scale * sum of the `dq_parts` dq32[part][row, d]) and, for the KEY-MAJOR
-// planes the backward kernel writes, (nplanes, B*H, key, query) with rows of L2 rounded up to 8 elements:
+// Backward epilogue, one launch: dq[row, d] = (dtype)(scale * dq32[row, d]) and, for the KEY-MAJOR
+// (dq32 == nullptr: dq has been written already) planes the backward kernel writes, (nplanes, B*H, key, query) with rows of L2 rounded up to 8 elements:
 // dbias_f32[bh][query][key] = sum_p planes[p][bh][key][query] in plane order, optional rounded copy
-int launch_bwd_epilogue(const float* dq32, int dq_parts, void* dq, const long long sdq[4], int B, int H, int L1, int L2, int D,
+int launch_bwd_epilogue(const float* dq32, void* dq, const long long sdq[4], int B, int H, int L1, int L2, int D,
                         float scale, const float* planes, int nplanes, float* dbias_f32, void* dbias_cast, bool bf16,
                         Status status, cudaStream_t stream);
 

@@ -31,7 +31,6 @@ FTA_NATIVE int native_mask_bias(const FtaProblem& prob, const FtaTensor4& bias, 
 // What fta_backward and fta_bwd_preprocess need in scratch memory for `prob`, planned once per call
 struct BackwardPlan {
   int nplanes;
-  int dq_parts;
   size_t workspace_bytes;  // of fta_backward
   size_t delta_bytes;      // of fta_bwd_preprocess's output
 };

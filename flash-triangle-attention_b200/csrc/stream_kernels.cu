@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(256) bwd_prologue_kernel(const uint16_t* __res
 // tiles few, a chain of dependent memory latencies: hence the small tile and eight planes in flight.
 // ------------------------------------------------------------------------------------------------
 template <int kD, bool kBf16, bool kDense>
-__global__ void __launch_bounds__(256) bwd_epilogue_kernel(const float* __restrict__ dq32, int dq_parts, uint16_t* __restrict__ dq,
+__global__ void __launch_bounds__(256) bwd_epilogue_kernel(const float* __restrict__ dq32, uint16_t* __restrict__ dq,
                                                            long long rows, int H, int L1, int L2, long long s_b,
                                                            long long s_h, long long s_i, long long s_j, float scale,
                                                            int dq_blocks, const float* __restrict__ planes, int nplanes,
@@ -499,14 +499,8 @@ __global__ void __launch_bounds__(256) bwd_epilogue_kernel(const float* __restri
          idx += nthreads) {
       const long long row = idx / LPR;
       const int part = static_cast<int>(idx % LPR);
-      float4 a = __ldg(reinterpret_cast<const float4*>(dq32 + row * kD + part * 8));
-      float4 c = __ldg(reinterpret_cast<const float4*>(dq32 + row * kD + part * 8 + 4));
-      if (dq_parts == 2) {
-        const float* second = dq32 + rows * kD + row * kD + part * 8;
-        const float4 a2 = __ldg(reinterpret_cast<const float4*>(second)), c2 = __ldg(reinterpret_cast<const float4*>(second + 4));
-        a = make_float4(a.x + a2.x, a.y + a2.y, a.z + a2.z, a.w + a2.w);
-        c = make_float4(c.x + c2.x, c.y + c2.y, c.z + c2.z, c.w + c2.w);
-      }
+      const float4 a = __ldg(reinterpret_cast<const float4*>(dq32 + row * kD + part * 8));
+      const float4 c = __ldg(reinterpret_cast<const float4*>(dq32 + row * kD + part * 8 + 4));
       long long oo;
       if constexpr (kDense) oo = row * kD + part * 8;
       else oo = strided_row_offset(row, H, L1, L2, s_b, s_h, s_i, s_j) + part * 8;
@@ -654,18 +648,18 @@ int launch_bwd_prologue(const void* bias, const long long sb[4], void* bias_t, i
   return static_cast<int>(cudaGetLastError());
 }
 
-int launch_bwd_epilogue(const float* dq32, int dq_parts, void* dq, const long long sdq[4], int B, int H, int L1, int L2, int D,
+int launch_bwd_epilogue(const float* dq32, void* dq, const long long sdq[4], int B, int H, int L1, int L2, int D,
                         float scale, const float* planes, int nplanes, float* dbias_f32, void* dbias_cast, bool bf16,
                         Status status, cudaStream_t stream) {
   const long long rows = static_cast<long long>(B) * H * L1 * L2;
-  const int dq_blocks = grid_for(rows * (D / 8), 256);
+  const int dq_blocks = dq32 ? grid_for(rows * (D / 8), 256) : 0;
   const int db_blocks = ((L2 + 31) / 32) * ((L2 + 31) / 32) * B * H;
   const int grid = dq_blocks + db_blocks;
   uint16_t* out = static_cast<uint16_t*>(dq);
   uint16_t* cast = static_cast<uint16_t*>(dbias_cast);
   const bool dense = is_dense(sdq, H, L1, L2, D);
   auto go = [&](auto kern) {
-    kern<<<grid, 256, 0, stream>>>(dq32, dq_parts, out, rows, H, L1, L2, sdq[0], sdq[1], sdq[2], sdq[3], scale, dq_blocks,
+    kern<<<grid, 256, 0, stream>>>(dq32, out, rows, H, L1, L2, sdq[0], sdq[1], sdq[2], sdq[3], scale, dq_blocks,
                                    planes, nplanes, B * H, dbias_f32, cast, status);
   };
   auto pick = [&](auto d_tag, auto bf_tag) {

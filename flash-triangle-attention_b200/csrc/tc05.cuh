@@ -218,11 +218,6 @@ __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* tmap, uint3
                ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* tmap, uint32_t src, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1), "r"(c2)
-               : "memory");
-}
 __device__ __forceinline__ void tma_reduce_add_3d_hint(const CUtensorMap* tmap, uint32_t src, int c0, int c1, int c2,
                                                        uint64_t pol) {
   asm volatile(
