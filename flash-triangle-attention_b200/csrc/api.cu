@@ -60,6 +60,16 @@ int map5(CUtensorMap* m, const FtaProblem* p, const FtaTensor5* t, uint32_t box_
   return fta::make_tmap_16bit(m, t->ptr, 5, dims, str, box, p->D * 2) == 0 ? FTA_OK : FTA_ERR_TENSOR_MAP;
 }
 
+// 5-D map over (D, L2, L1, H, B) for stores of 32 rows x 32 columns
+int map5_out(CUtensorMap* m, const FtaProblem* p, const FtaTensor5* t) {
+  const uint64_t dims[5] = {static_cast<uint64_t>(p->D), static_cast<uint64_t>(p->L2), static_cast<uint64_t>(p->L1),
+                            static_cast<uint64_t>(p->H), static_cast<uint64_t>(p->B)};
+  const uint64_t str[5] = {0, static_cast<uint64_t>(t->stride[3]) * 2, static_cast<uint64_t>(t->stride[2]) * 2,
+                           static_cast<uint64_t>(t->stride[1]) * 2, static_cast<uint64_t>(t->stride[0]) * 2};
+  const uint32_t box[5] = {32, 32, 1, 1, 1};
+  return fta::make_tmap_16bit(m, t->ptr, 5, dims, str, box, 64) == 0 ? FTA_OK : FTA_ERR_TENSOR_MAP;
+}
+
 int padded_l2(const FtaProblem* p) { return (p->L2 + 127) / 128 * 128; }
 
 // 4-D map over the bias (key, query, H, B); `box_k` keys x 128 queries per tile. The bias the kernels
@@ -180,7 +190,8 @@ int backward(const FtaProblem* prob, int nplanes, const fta::PreArgs* pre, const
   bt.stride[3] = 1;
   // the backward kernel loads Q and dO by 64-query halves
   if ((rc = map5(&a.tmQ, prob, q, 64)) || (rc = map5(&a.tmK, prob, k)) || (rc = map5(&a.tmV, prob, v)) ||
-      (rc = map5(&a.tmDO, prob, dout, 64)) || (rc = map_bias(&a.tmBiasT, prob, &bt, 64, 128)))
+      (rc = map5(&a.tmDO, prob, dout, 64)) || (rc = map5_out(&a.tmDK, prob, dk)) || (rc = map5_out(&a.tmDV, prob, dv)) ||
+      (rc = map5_out(&a.tmDQ16, prob, dq)) || (rc = map_bias(&a.tmBiasT, prob, &bt, 64, 128)))
     return rc;
   {
     // dq32 seen as (B*H*L1, L2, D) float32; the kernel adds 32-query x 16-column tiles into it with
@@ -201,9 +212,6 @@ int backward(const FtaProblem* prob, int nplanes, const fta::PreArgs* pre, const
   a.lse = lse;
   a.delta = delta;
   a.dq32 = dq32;
-  a.dq = dq->ptr;
-  a.dk = dk->ptr;
-  a.dv = dv->ptr;
   a.status = status.word;
   a.nplanes = nplanes;
   a.B = prob->B;
@@ -214,9 +222,6 @@ int backward(const FtaProblem* prob, int nplanes, const fta::PreArgs* pre, const
   a.bf16 = bf16;
   long long sdq[4];
   for (int i = 0; i < 4; ++i) {
-    a.sdq[i] = dq->stride[i];
-    a.sdk[i] = dk->stride[i];
-    a.sdv[i] = dv->stride[i];
     sdq[i] = dq->stride[i];
   }
   a.sm_scale = sm_scale;

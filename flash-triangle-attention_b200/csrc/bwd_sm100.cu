@@ -110,13 +110,9 @@ struct BwdParams {
   const float* lse;  // three planes: -max (natural-log units), -log2(sum), c (see the forward kernel)
   const float* delta;
   float* dq32;
-  void* dq;  // written by the kernel itself where L2 <= 128
-  void* dk;
-  void* dv;
   int* status;
   int H, L1, L2, NP, BH;
   int stat_pitch;  // row pitch of lse / delta: L2 rounded up to 128
-  long long sdq[4], sdk[4], sdv[4];
   float scale;  // sm_scale
   long long stat_stride;  // elements between the statistics planes
 };
@@ -133,7 +129,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                const __grid_constant__ CUtensorMap tmBiasT, const __grid_constant__ CUtensorMap tmDQ,
-               const __grid_constant__ CUtensorMap tmPlane, const BwdParams p) {
+               const __grid_constant__ CUtensorMap tmPlane, const __grid_constant__ CUtensorMap tmDK,
+               const __grid_constant__ CUtensorMap tmDV, const __grid_constant__ CUtensorMap tmDQ16, const BwdParams p) {
   using C = BwdCfg<kD>;
   constexpr int G = C::G;
   extern __shared__ uint8_t smem_raw[];
@@ -216,6 +213,8 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         tma_prefetch_desc(&tmBiasT);
         tma_prefetch_desc(&tmDQ);
         tma_prefetch_desc(&tmPlane);
+        tma_prefetch_desc(&tmDK);
+        tma_prefetch_desc(&tmDV);
       }
       // K/V/Q/dO tiles stream through L2 (each is read within a short window and never again);
       // the bias tiles are re-read by every group and stay
@@ -459,21 +458,37 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // rows per warp, into the float32 accumulator with TMA reductions), and dK / dV of a row after its
     // last query block. Every warp handles its own 32 TMEM lanes from end to end, so the four need no barrier.
     reg_dec<kRegsDrain>();
-    const int lrow = (warp & 3) * 32 + lane;  // TMEM lane: query row of a dQ tile, key row of dK / dV
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const int row0 = (warp & 3) * 32;  // first TMEM lane: query row of a dQ tile, key row of dK / dV
     const uint32_t stage = smem_u32(sDQ) + (warp & 3) * 2048;
-    const bool key_live = kb * 128 + lrow < p.L2;  // keys past L2 in a ragged block own no output row
-    // 16 columns of this thread's row, scaled and rounded
-    auto store16 = [&](uint16_t* out, const uint32_t (&x)[16], float mul) {
+    // 32 columns of this warp's 32 rows, scaled and rounded, through the staging rows (64-byte swizzle) to a box of an
+    // output tensor, clipped by its map. Not from registers: stores that find the SM's way out full, as it is when
+    // dBias boxes are leaving, hold up the shared-memory accesses of the compute warps behind them.
+    // `free_bar`: arrived at once TMEM has been read (0: none).
+    auto emit = [&](uint32_t taddr, const CUtensorMap* map, int col, int row, int irow, float mul, uint32_t free_bar) {
+      uint32_t x[16], pk[16];
 #pragma unroll
-      for (int v4 = 0; v4 < 2; ++v4) {
-        uint4 ov;
-        ov.x = pack2<kBf16>(__uint_as_float(x[v4 * 8 + 0]) * mul, __uint_as_float(x[v4 * 8 + 1]) * mul);
-        ov.y = pack2<kBf16>(__uint_as_float(x[v4 * 8 + 2]) * mul, __uint_as_float(x[v4 * 8 + 3]) * mul);
-        ov.z = pack2<kBf16>(__uint_as_float(x[v4 * 8 + 4]) * mul, __uint_as_float(x[v4 * 8 + 5]) * mul);
-        ov.w = pack2<kBf16>(__uint_as_float(x[v4 * 8 + 6]) * mul, __uint_as_float(x[v4 * 8 + 7]) * mul);
-        if (key_live) *reinterpret_cast<uint4*>(out + v4 * 8) = ov;
+      for (int half = 0; half < 2; ++half) {
+        tmem_ld16(taddr + col + half * 16 + lane_off, x);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          pk[half * 8 + e] = pack2<kBf16>(__uint_as_float(x[2 * e]) * mul, __uint_as_float(x[2 * e + 1]) * mul);
       }
+      if (elect_one()) bulk_wait_read_all();  // this warp's previous transfer has read the staging rows
+      if (free_bar) tc_fence_before_sync();
+      __syncwarp();
+      if (free_bar && lane == 0) mbar_arrive(free_bar);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        st_shared_v4(stage + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4), pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (elect_one()) {
+        tma_store_5d(map, stage, col, row, irow, h, b);
+        bulk_commit_group();
+      }
+      __syncwarp();
     };
     bool ok = true;
     int tt = 0;
@@ -486,6 +501,11 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           ok = mbar_wait_warp(bar(C::B_DQDONE + buf), (tt >> 1) & 1, w, 0x46);
           if (!ok) break;
           tc_fence_after_sync();
+          if (nkb == 1) {
+#pragma unroll 1
+            for (int c = 0; c < kD; c += 32)
+              emit(tbase + C::TM_DQ + buf * kD, &tmDQ16, c, row0, i0 + g, p.scale, c + 32 == kD ? bar(C::B_DQFREE + buf) : 0u);
+          } else {
 #pragma unroll 1
           for (int c = 0; c < kD / 16; ++c) {
             uint32_t qv[16];
@@ -495,11 +515,6 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             if (c == kD / 16 - 1) tc_fence_before_sync();
             __syncwarp();
             if (c == kD / 16 - 1 && lane == 0) mbar_arrive(bar(C::B_DQFREE + buf));
-            if (nkb == 1) {
-              store16(reinterpret_cast<uint16_t*>(p.dq) + b * p.sdq[0] + h * p.sdq[1] + static_cast<long long>(i0 + g) * p.sdq[2] +
-                          static_cast<long long>(lrow) * p.sdq[3] + c * 16, qv, p.scale);
-              continue;
-            }
 #pragma unroll
             for (int j = 0; j < 4; ++j)  // 64-byte swizzle
               st_shared_v4(stage + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4), qv[4 * j], qv[4 * j + 1], qv[4 * j + 2],
@@ -507,32 +522,21 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             fence_proxy_async_smem();
             __syncwarp();
             if (elect_one()) {
-              tma_reduce_add_3d(&tmDQ, stage, c * 16, jb * 128 + (warp & 3) * 32, bh * p.L1 + i0 + g);
+              tma_reduce_add_3d(&tmDQ, stage, c * 16, jb * 128 + row0, bh * p.L1 + i0 + g);
               bulk_commit_group();
             }
             __syncwarp();
+          }
           }
           if (jb == nq - 1) {
             ok = mbar_wait_warp(bar(C::B_ACCFULL + g), n & 1, w, 0x45);
             if (!ok) break;
             tc_fence_after_sync();
 #pragma unroll 1
-            for (int c = 0; c < 2 * kD / 16; ++c) {  // dK (scaled by sm_scale, flash_tt_attn.py:518), then dV
-              const bool is_dv = c >= kD / 16;
-              const long long* sd = is_dv ? p.sdv : p.sdk;
-              uint16_t* optr = reinterpret_cast<uint16_t*>(is_dv ? p.dv : p.dk) + b * sd[0] + h * sd[1] +
-                               static_cast<long long>(i0 + g) * sd[2] + static_cast<long long>(kb * 128 + lrow) * sd[3] +
-                               (c & (kD / 16 - 1)) * 16;
-              const float mul = is_dv ? 1.0f : p.scale;
-              uint32_t av[16];
-              tmem_ld16(tbase + C::TM_ACC + g * 2 * kD + c * 16 + lane_off, av);
-              tmem_ld_wait();
-              if (c == 2 * kD / 16 - 1) {
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(C::B_ACCFREE + g));
-              }
-              store16(optr, av, mul);
+            for (int c = 0; c < 2 * kD; c += 32) {  // dK (scaled by sm_scale, flash_tt_attn.py:518), then dV
+              const bool is_dv = c >= kD;
+              emit(tbase + C::TM_ACC + g * 2 * kD + (is_dv ? kD : 0), is_dv ? &tmDV : &tmDK, c & (kD - 1), kb * 128 + row0, i0 + g,
+                   is_dv ? 1.0f : p.scale, c + 32 == 2 * kD ? bar(C::B_ACCFREE + g) : 0u);
             }
           }
         }
@@ -731,25 +735,18 @@ int launch_bwd_t(const BwdArgs& a, int NP, cudaStream_t stream) {
   p.lse = a.lse;
   p.delta = a.delta;
   p.dq32 = a.dq32;
-  p.dq = a.dq;
-  p.dk = a.dk;
-  p.dv = a.dv;
   p.status = a.status;
   p.H = a.H;
   p.L1 = a.L1;
   p.L2 = a.L2;
   p.NP = NP;
   p.BH = a.B * a.H;
-  for (int i = 0; i < 4; ++i) {
-    p.sdq[i] = a.sdq[i];
-    p.sdk[i] = a.sdk[i];
-    p.sdv[i] = a.sdv[i];
-  }
   p.scale = a.sm_scale;
   p.stat_pitch = (a.L2 + 127) / 128 * 128;
   p.stat_stride = static_cast<long long>(a.B) * a.H * a.L1 * p.stat_pitch;
   const int grid = a.B * a.H * NP * ((a.L2 + 127) / 128);
-  kern<<<grid, kBwdThreads, C::SMEM_BYTES, stream>>>(a.tmQ, a.tmK, a.tmV, a.tmDO, a.tmBiasT, a.tmDQ, a.tmPlane, p);
+  kern<<<grid, kBwdThreads, C::SMEM_BYTES, stream>>>(a.tmQ, a.tmK, a.tmV, a.tmDO, a.tmBiasT, a.tmDQ, a.tmPlane, a.tmDK,
+                                                    a.tmDV, a.tmDQ16, p);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -94,18 +94,15 @@ int fwd_rows_per_cta(int D);
 struct BwdArgs {
   CUtensorMap tmQ, tmK, tmV, tmDO, tmBiasT;  // tmBiasT: over the key-major copy of the bias
   CUtensorMap tmDQ;    // dq32 as a 3-D float32 tensor (B*H*L1, L2, D), box 128 queries x 32 columns, 128 B swizzle
+  CUtensorMap tmDK, tmDV, tmDQ16;  // the 16-bit outputs, boxes of 32 columns x 32 rows, 64 B swizzle (tmDQ16: L2 <= 128)
   CUtensorMap tmPlane; // the partial dBias planes as (nplanes*B*H, L2 keys, L2 queries) float32, same box
   const float* lse;    // (3,B,H,L1,L2): -max, -log2(sum), combined (NaN where inexact)
   const float* delta;  // (B,H,L1,L2)
   float* dq32;         // (B,H,L1,L2,D) float32, zeroed; receives sum over key blocks of dS K (not used for L2 <= 128)
-  void* dq;            // written where L2 <= 128
-  void* dk;
-  void* dv;
   int* status;
   int B, H, L1, L2, D;
   int nplanes;  // bwd_num_planes()
   bool bf16;
-  long long sdq[4], sdk[4], sdv[4];  // element strides of dQ, dK, dV over (B, H, L1, L2)
   float sm_scale;
 };
 int launch_bwd(const BwdArgs& a, cudaStream_t stream);
