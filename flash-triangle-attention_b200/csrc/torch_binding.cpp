@@ -10,6 +10,7 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include <cstdio>
@@ -242,6 +243,8 @@ void require(bool ok, const char* msg) {
 
 void check_arguments(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& bias,
                      const std::optional<at::Tensor>& key_mask) {
+  // a trace would record the allocation of O and not the launches that fill it
+  require(!torch::jit::tracer::isTracing(), "flash_tt_attn.attention cannot be recorded by torch.jit.trace");
   require(q.dim() == 5 && q.size(4) == k.size(-1) && k.size(-1) == v.size(-1), "q, k, v must be 5-D with one head dimension");
   require(q.size(4) == 32 || q.size(4) == 64, "head dimension must be 32 or 64");
   const auto dt = q.scalar_type();

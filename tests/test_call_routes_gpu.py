@@ -1,0 +1,24 @@
+"""Ways of calling ``attention()`` in which the launches are not seen by the caller's machinery: what cannot be done
+is refused, nothing is answered from memory that no kernel has written."""
+import pytest
+import torch
+
+import flash_tt_attn as fta
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(L2=128, dtype=torch.float16, L1=2, D=32):
+    g = torch.Generator(device="cuda").manual_seed(L2)
+    r = lambda *s: torch.randn(s, device="cuda", dtype=dtype, generator=g)
+    return [r(1, 1, L1, L2, D) for _ in range(3)] + [r(1, 1, L2, L2)]
+
+
+@pytest.mark.parametrize("grad", [False, True])
+def test_jit_trace_is_refused(grad):
+    q, k, v, b = _inputs()
+    q.requires_grad_(grad)
+    with pytest.raises(AssertionError, match="torch.jit.trace"):
+        torch.jit.trace(lambda *a: fta.attention(*a, 0.2), (q, k, v, b), check_trace=False)
+    assert torch.isfinite(fta.attention(q, k, v, b, 0.2)).all()  # the tracer is gone again
+    fta.check_device_status()
