@@ -260,12 +260,17 @@ void check_arguments(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
   ensure_status(q.device());
 }
 
+bool has_tangent(const at::Tensor& t) { return t._fw_grad(/*level=*/0).defined(); }
+
 at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& bias,
                      double sm_scale, const std::optional<at::Tensor>& key_mask) {
   check_arguments(q, k, v, bias, key_mask);
   const bool keep = at::GradMode::is_enabled() &&
                     (q.requires_grad() || k.requires_grad() || v.requires_grad() || bias.requires_grad());
-  if (!keep) return run_forward(q, k, v, bias, sm_scale, key_mask, false).o;
+  // A forward-mode tangent on any input goes through the autograd function whatever the mode: it has no formula for
+  // tangents and says so, where the bare pass would drop them.
+  const bool dual = has_tangent(q) || has_tangent(k) || has_tangent(v) || has_tangent(bias);
+  if (!keep && !dual) return run_forward(q, k, v, bias, sm_scale, key_mask, false).o;
   return Attention::apply(q, k, v, bias, sm_scale, key_mask);
 }
 

@@ -22,3 +22,19 @@ def test_jit_trace_is_refused(grad):
         torch.jit.trace(lambda *a: fta.attention(*a, 0.2), (q, k, v, b), check_trace=False)
     assert torch.isfinite(fta.attention(q, k, v, b, 0.2)).all()  # the tracer is gone again
     fta.check_device_status()
+
+
+@pytest.mark.parametrize("which", range(4))
+@pytest.mark.parametrize("mode", ["no_leaf", "leaf", "no_grad"])
+def test_forward_mode_tangents_are_refused_not_dropped(which, mode):
+    import torch.autograd.forward_ad as fwad
+    t = _inputs()
+    if mode == "leaf":
+        t[0].requires_grad_()
+    with fwad.dual_level(), torch.set_grad_enabled(mode != "no_grad"):
+        args = list(t)
+        args[which] = fwad.make_dual(t[which], torch.ones_like(t[which]))
+        with pytest.raises((RuntimeError, NotImplementedError), match="jvp"):
+            fta.attention(*args, 0.2)
+        assert torch.isfinite(fta.attention(*t, 0.2)).all()  # no tangent, no objection
+    fta.check_device_status()
