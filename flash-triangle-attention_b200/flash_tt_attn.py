@@ -315,6 +315,12 @@ def _block_sizes(L1: int, block_rows: int):
     return sizes + ramp[::-1]
 
 
+def _blocks_workspace_bytes(B, H, L2, D, dtype_code, sizes):
+    """Backward workspace that serves every block of ``sizes`` rows. Not that of the largest block: a shorter one
+    may be given more dBias planes (B1 H1 L256 D64: 48 for 96 rows, 64 for 64) and need more."""
+    return max(int(_cabi.lib().fta_bwd_workspace_bytes(FtaProblem(B, H, n, L2, D, dtype_code))) for n in set(sizes))
+
+
 def _copy_rows(lib, dst, dst_row0, src, src_row0, nrows, stream):
     """Rows [row0, row0 + nrows) of the L1 axis of every (b, h): one strided transfer. Both tensors
     are (B, H, *, L2, D) and dense in their last two axes and across (b, h)."""
@@ -372,7 +378,7 @@ def attention_fwd_bwd_streamed(host, sm_scale, out, block_rows=96, device=None, 
         slots = [{**{k: mk(B, H, cap, L2, D) for k in names_in + names_out}, "ores": mk(B, H, cap, L2, D),
                   "lse": mk(3, B, H, cap, L2p, dtype=torch.float32), "delta": mk(B, H, cap, L2p, dtype=torch.float32)}
                  for _ in range(NSLOT)]
-        ws_bytes = int(L.fta_bwd_workspace_bytes(FtaProblem(B, H, cap, L2, D, dtype_code)))
+        ws_bytes = _blocks_workspace_bytes(B, H, L2, D, dtype_code, sizes)
         ws = mk(ws_bytes, dtype=torch.uint8)
         ev_in = [torch.cuda.Event() for _ in range(NSLOT)]
         ev_comp = [torch.cuda.Event() for _ in range(NSLOT)]

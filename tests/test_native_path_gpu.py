@@ -85,3 +85,26 @@ def test_backward_is_bit_reproducible_over_many_blocks(D, L1, L2):
         assert torch.equal(torch.cat([p[i] for p in parts], dim=2), first[i])
     assert torch.allclose(parts[0][3] + parts[1][3], first[3], atol=1e-4, rtol=1e-5)
     fta.check_device_status()
+
+
+@pytest.mark.parametrize("B,H,L1,L2,D", [(1, 1, 256, 256, 64), (1, 4, 300, 576, 32)])
+def test_streamed_call_with_blocks_that_need_more_scratch_than_the_largest(B, H, L1, L2, D):
+    """Default blocks, where a short block is split over more dBias planes than a full one: accepted, and equal to
+    the call on device tensors (dQ and dBias: float32 sums whose order may differ)."""
+    g = torch.Generator().manual_seed(L2)
+    host = {n: torch.randn(B, H, L1, L2, D, generator=g).bfloat16().pin_memory() for n in ("q", "k", "v", "do")}
+    host["bias"] = torch.randn(B, H, L2, L2, generator=g).bfloat16().pin_memory()
+    out = {n: torch.full_like(host["q"], float("nan")).pin_memory() for n in ("o", "dq", "dk", "dv")}
+    out["dbias"] = torch.empty_like(host["bias"]).pin_memory()
+    fta.attention_fwd_bwd_streamed(host, 0.2, out)
+    db32 = fta.last_dbias_f32().clone()
+    leaves = [host[n].cuda().requires_grad_() for n in ("q", "k", "v", "bias")]
+    o = fta.attention(*leaves, 0.2)
+    o.backward(host["do"].cuda())
+    fta.check_device_status()
+    assert torch.equal(out["o"], o.detach().cpu())
+    assert torch.equal(out["dk"], leaves[1].grad.cpu()) and torch.equal(out["dv"], leaves[2].grad.cpu())
+    # one bf16 ulp of the largest value
+    assert float((out["dq"].float() - leaves[0].grad.cpu().float()).abs().max()) <= float(out["dq"].float().abs().max()) * 2.0 ** -8
+    ref = fta.last_dbias_f32()
+    assert float((db32 - ref).abs().max()) <= 1e-4 * float(ref.abs().max()) + 1e-5
