@@ -83,12 +83,20 @@ class _Status:
                                "in an earlier call; its outputs are incomplete)")
 
 
+def _indexed(device) -> torch.device:
+    """``device`` with an index: "cuda" alone is the current device."""
+    device = torch.device(device)
+    return torch.device(device.type, torch.cuda.current_device()) if device.index is None else device
+
+
 def _status_of(device) -> _Status:
+    device = _indexed(device)
     key = (device.type, device.index)
     st = _status_words.get(key)
     if st is None:
-        st = _status_words[key] = _Status(device)
+        st = _Status(device)
         _native().set_status(device.index, st.word, st.mirror)
+        _status_words[key] = st
     return st
 
 
@@ -99,8 +107,7 @@ def _status(device) -> torch.Tensor:
 def check_device_status(device=None) -> None:
     """Raise if a kernel of this module reported a device-side error (a bounded wait that ran
     out). Synchronises the device's current stream."""
-    device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    st = _status_of(device)
+    st = _status_of("cuda" if device is None else device)
     st.raise_if_set(int(st.word.item()))
 
 
@@ -351,7 +358,7 @@ def attention_fwd_bwd_streamed(host, sm_scale, out, block_rows=96, device=None, 
     group: with a process group, ``host`` holds this rank's rows and dBias is all-reduced once.
     Returns after everything has arrived in ``out``.
     """
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+    dev = _indexed("cuda" if device is None else device)
     q_h, b_h = host["q"], host["bias"]
     B, H, L1, L2, D = q_h.shape
     assert L2 % 8 == 0 and D in (32, 64) and q_h.dtype in (torch.float16, torch.bfloat16)

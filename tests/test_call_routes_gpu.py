@@ -38,3 +38,18 @@ def test_forward_mode_tangents_are_refused_not_dropped(which, mode):
             fta.attention(*args, 0.2)
         assert torch.isfinite(fta.attention(*t, 0.2)).all()  # no tangent, no objection
     fta.check_device_status()
+
+
+def test_device_cuda_names_the_word_the_kernels_write():
+    q, k, v, b = _inputs()
+    fta.attention(q, k, v, b, 0.2)
+    fta.check_device_status("cuda")
+    host = {n: torch.randn(1, 1, 5, 128, 32).bfloat16().pin_memory() for n in ("q", "k", "v", "do")}
+    host["bias"] = torch.randn(1, 1, 128, 128).bfloat16().pin_memory()
+    out = {n: torch.empty_like(host["q"]).pin_memory() for n in ("o", "dq", "dk", "dv")}
+    out["dbias"] = torch.empty_like(host["bias"]).pin_memory()
+    fta.attention_fwd_bwd_streamed(host, 0.2, out, device="cuda")
+    fta._status_of(q.device).word.fill_(0x1042)
+    with pytest.raises(RuntimeError, match="0x1042"):
+        fta.check_device_status("cuda")
+    fta.check_device_status("cuda")

@@ -124,3 +124,48 @@ def test_streamed_workspace_serves_every_block():
         assert 0 < max(need.values()) <= have
         not_the_largest += need[max(sizes)] < have
     assert not_the_largest >= 2  # the case this is about is among them
+
+
+class _FakeNative:
+    def __init__(self):
+        self.calls = []
+
+    def set_status(self, index, word, mirror):
+        assert isinstance(index, int)
+        self.calls.append((index, word, mirror))
+
+
+@pytest.fixture
+def fake_device(monkeypatch):
+    """The status bookkeeping with CPU tensors in the place of a device's."""
+    class FakeStatus(fta._Status):
+        def __init__(self, device):
+            self.word, self.mirror = torch.zeros(1, dtype=torch.int32), torch.zeros(1, dtype=torch.int32)
+
+    native = _FakeNative()
+    monkeypatch.setattr(fta, "_native", lambda: native)
+    monkeypatch.setattr(fta, "_Status", FakeStatus)
+    monkeypatch.setattr(fta, "_status_words", {})
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    return native
+
+
+def test_a_device_without_an_index_is_the_current_one(fake_device):
+    """The word that attention() registers for cuda:3 is the one that "cuda" names while device 3 is current."""
+    st = fta._status_of(torch.device("cuda", 3))
+    assert fta._status_of(torch.device("cuda")) is st and fta._status_of("cuda") is st
+    assert [c[0] for c in fake_device.calls] == [3]
+    fta.check_device_status("cuda")
+    st.word.fill_(0x1042)
+    with pytest.raises(RuntimeError, match="0x1042"):
+        fta.check_device_status("cuda")
+    fta.check_device_status()
+
+
+def test_a_status_word_is_kept_only_once_it_is_registered(fake_device, monkeypatch):
+    def fails(*a):
+        raise RuntimeError("not registered")
+    monkeypatch.setattr(fake_device, "set_status", fails)
+    with pytest.raises(RuntimeError, match="not registered"):
+        fta._status_of("cuda")
+    assert not fta._status_words
