@@ -30,6 +30,7 @@ There is no fallback: without a CUDA device and a built ``libfta.so`` every call
 from __future__ import annotations
 
 import os
+import threading
 
 import torch
 
@@ -42,6 +43,7 @@ __all__ = ["attention", "attention_fwd_bwd_streamed", "reference_tt_attn", "chec
 _DEBUG = os.environ.get("FTA_DEBUG", "0") == "1"
 _SAVE_O_RESIDUAL = os.environ.get("FTA_SAVE_O_RESIDUAL", "1") != "0"
 _status_words = {}
+_status_lock = threading.RLock()
 _copy_streams = {}
 _ext = None
 
@@ -94,9 +96,12 @@ def _status_of(device) -> _Status:
     key = (device.type, device.index)
     st = _status_words.get(key)
     if st is None:
-        st = _Status(device)
-        _native().set_status(device.index, st.word, st.mirror)
-        _status_words[key] = st
+        with _status_lock:  # threads that meet a device together: one word, kernels in flight write to it
+            st = _status_words.get(key)
+            if st is None:
+                st = _Status(device)
+                _native().set_status(device.index, st.word, st.mirror)
+                _status_words[key] = st
     return st
 
 

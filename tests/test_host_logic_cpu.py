@@ -169,3 +169,29 @@ def test_a_status_word_is_kept_only_once_it_is_registered(fake_device, monkeypat
     with pytest.raises(RuntimeError, match="not registered"):
         fta._status_of("cuda")
     assert not fta._status_words
+
+
+def test_threads_that_meet_a_device_together_share_one_status_word(fake_device, monkeypatch):
+    """A second word for the device would replace the first, which kernels of the other thread still write to."""
+    import threading
+    import time
+    slow = fta._Status
+
+    class SlowStatus(slow):
+        def __init__(self, device):
+            time.sleep(0.05)  # as an allocation does, this lets the other threads in
+            super().__init__(device)
+
+    monkeypatch.setattr(fta, "_Status", SlowStatus)
+    got, start = [], threading.Barrier(8)
+
+    def meet():
+        start.wait()
+        got.append(fta._status_of("cuda"))
+
+    threads = [threading.Thread(target=meet) for _ in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(got) == 8 and all(st is got[0] for st in got) and len(fake_device.calls) == 1
