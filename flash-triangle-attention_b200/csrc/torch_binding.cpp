@@ -36,6 +36,18 @@ bool g_save_o_residual = true;
 at::Tensor g_last_dbias_f32;  // of the most recent backward call, any thread
 std::mutex g_last_mu;
 
+// What was there before dies after the lock is given back: if Python has seen that tensor, its end takes the
+// interpreter's lock, which a thread that waits for ours may hold.
+void set_last_dbias_f32(at::Tensor t) {
+  std::lock_guard<std::mutex> lock(g_last_mu);
+  std::swap(t, g_last_dbias_f32);
+}
+std::optional<at::Tensor> last_dbias_f32() {
+  std::lock_guard<std::mutex> lock(g_last_mu);
+  if (!g_last_dbias_f32.defined()) return std::nullopt;
+  return g_last_dbias_f32;
+}
+
 // Called with a device index the first time attention() meets that device: has the Python module create
 // and register its status word. Never released (it lives as long as the interpreter).
 py::object* g_make_status = nullptr;
@@ -212,10 +224,7 @@ BackwardOut run_backward(const at::Tensor& q, const at::Tensor& k, const at::Ten
                                 static_cast<const float*>(saved.data_ptr()), static_cast<float>(sm_scale), v5(r.dq),
                                 v5(r.dk), v5(r.dv), r.dbias_f32.data_ptr<float>(), cast ? r.dbias.data_ptr() : nullptr,
                                 ws.data_ptr(), st.pair, stream), "fta_backward");
-  {
-    std::lock_guard<std::mutex> lock(g_last_mu);
-    g_last_dbias_f32 = r.dbias_f32;
-  }
+  set_last_dbias_f32(r.dbias_f32);
   return r;
 }
 
@@ -288,16 +297,6 @@ py::tuple backward_pass(const at::Tensor& q, const at::Tensor& k, const at::Tens
   return py::make_tuple(r.dq, r.dk, r.dv, r.dbias, r.dbias_f32);
 }
 
-std::optional<at::Tensor> last_dbias_f32() {
-  std::lock_guard<std::mutex> lock(g_last_mu);
-  if (!g_last_dbias_f32.defined()) return std::nullopt;
-  return g_last_dbias_f32;
-}
-void set_last_dbias_f32(at::Tensor t) {
-  std::lock_guard<std::mutex> lock(g_last_mu);
-  g_last_dbias_f32 = std::move(t);
-}
-
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -311,8 +310,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("set_last_dbias_f32", &set_last_dbias_f32);
   // the saved tensor must not outlive the allocator it came from
   py::module_::import("atexit").attr("register")(py::cpp_function([] {
-    std::lock_guard<std::mutex> lock(g_last_mu);
-    g_last_dbias_f32 = at::Tensor();
+    set_last_dbias_f32(at::Tensor());
     for (auto& s : g_status) s = DeviceStatus();
   }));
 }

@@ -195,3 +195,48 @@ def test_threads_that_meet_a_device_together_share_one_status_word(fake_device, 
     for t in threads:
         t.join()
     assert len(got) == 8 and all(st is got[0] for st in got) and len(fake_device.calls) == 1
+
+
+_LAST_DBIAS = r"""
+import os, sys, threading, weakref
+sys.path.insert(0, {root!r}); sys.path.insert(0, os.path.join({root!r}, "flash-triangle-attention_b200"))
+import torch
+import flash_tt_attn as fta
+ext = fta._native()
+seen = []
+
+def hold():  # a tensor whose Python side is finalised when the library lets go of it
+    t = torch.zeros(3)
+    weakref.finalize(t, lambda: seen.append(fta.last_dbias_f32().numel()))
+    ext.set_last_dbias_f32(t)
+
+for n in range(3):
+    hold()
+assert len(seen) == 2, seen
+stop = []
+
+def look():
+    while not stop:
+        fta.last_dbias_f32()
+
+threads = [threading.Thread(target=look) for _ in range(3)]
+for t in threads:
+    t.start()
+for n in range(300):
+    hold()
+stop.append(1)
+for t in threads:
+    t.join()
+print("through", flush=True)
+"""
+
+
+def test_last_dbias_lets_go_of_the_old_tensor_outside_its_lock(tmp_path):
+    """Letting go of a tensor that Python has seen runs the interpreter (its lock, its finalisers). Under the lock
+    of ``last_dbias_f32()`` that is a deadlock with whoever holds the interpreter and waits for that lock; here a
+    finaliser asks for it. In a process of its own, which ends by itself unless it is stuck."""
+    script = tmp_path / "last_dbias.py"
+    script.write_text(_LAST_DBIAS.format(root=ROOT))
+    r = subprocess.run([sys.executable, str(script)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True,
+                       timeout=120)
+    assert r.returncode == 0 and "through" in r.stdout, r.stdout
