@@ -274,6 +274,7 @@ bool has_tangent(const at::Tensor& t) { return t._fw_grad(/*level=*/0).defined()
 at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& bias,
                      double sm_scale, const std::optional<at::Tensor>& key_mask) {
   check_arguments(q, k, v, bias, key_mask);
+  py::gil_scoped_release no_gil;  // as torch's own operators do: an allocation or a full launch queue may wait
   const bool keep = at::GradMode::is_enabled() &&
                     (q.requires_grad() || k.requires_grad() || v.requires_grad() || bias.requires_grad());
   // A forward-mode tangent on any input goes through the autograd function whatever the mode: it has no formula for
@@ -287,13 +288,21 @@ at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
 py::tuple forward_pass(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& bias,
                        double sm_scale, const std::optional<at::Tensor>& key_mask) {
   check_arguments(q, k, v, bias, key_mask);
-  ForwardOut r = run_forward(q, k, v, bias, sm_scale, key_mask, true);
+  ForwardOut r;
+  {
+    py::gil_scoped_release no_gil;
+    r = run_forward(q, k, v, bias, sm_scale, key_mask, true);
+  }
   return py::make_tuple(r.q, r.k, r.v, r.bias, r.o, r.saved);
 }
 py::tuple backward_pass(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& bias,
                         const at::Tensor& o, const at::Tensor& saved, const at::Tensor& dout, double sm_scale, bool cast) {
   require(dout.scalar_type() == q.scalar_type(), "the gradient of O must have O's dtype");
-  BackwardOut r = run_backward(q, k, v, bias, o, saved, dout, sm_scale, cast);
+  BackwardOut r;
+  {
+    py::gil_scoped_release no_gil;
+    r = run_backward(q, k, v, bias, o, saved, dout, sm_scale, cast);
+  }
   return py::make_tuple(r.dq, r.dk, r.dv, r.dbias, r.dbias_f32);
 }
 

@@ -53,3 +53,52 @@ def test_device_cuda_names_the_word_the_kernels_write():
     with pytest.raises(RuntimeError, match="0x1042"):
         fta.check_device_status("cuda")
     fta.check_device_status("cuda")
+
+
+
+@pytest.mark.parametrize("route", ["attention", "forward_pass", "backward_pass"])
+def test_other_threads_run_while_a_pass_waits_in_native_code(route):
+    """Behind a kernel of half a second the launch queue fills up and a launch waits for room. Meanwhile a second
+    thread must have the interpreter: its longest pause is a fraction of that wait."""
+    import threading
+    import time
+    ext = fta._native()
+    q, k, v, b = _inputs()
+    fta.attention(q, k, v, b, 0.2)
+    state = ext.forward_pass(q, k, v, b, 0.2, None)
+    dout = torch.ones_like(q)
+    call = {"attention": lambda: fta.attention(q, k, v, b, 0.2),
+            "forward_pass": lambda: ext.forward_pass(q, k, v, b, 0.2, None),
+            "backward_pass": lambda: ext.backward_pass(*state, dout, 0.2, True)}[route]
+    call()
+    torch.cuda.synchronize()
+    pause, waiting, stop = [0.0], [], []
+
+    def other():
+        last = time.perf_counter()
+        while not stop:
+            time.sleep(0.001)
+            now = time.perf_counter()
+            if waiting:
+                pause[0] = max(pause[0], now - last)
+            last = now
+
+    thread = threading.Thread(target=other)
+    thread.start()
+    try:
+        time.sleep(0.05)
+        waiting.append(1)
+        torch.cuda._sleep(1_000_000_000)  # cycles: about half a second
+        longest = 0.0
+        for _ in range(2000):
+            t = time.perf_counter()
+            call()
+            longest = max(longest, time.perf_counter() - t)
+        time.sleep(0.01)
+    finally:
+        stop.append(1)
+        thread.join()
+    fta.check_device_status()
+    if longest < 0.1:
+        pytest.skip(f"no launch had to wait (longest call {longest * 1e3:.1f} ms)")
+    assert pause[0] < 0.5 * longest, (pause[0], longest)
