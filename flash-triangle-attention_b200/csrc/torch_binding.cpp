@@ -61,22 +61,31 @@ void set_status(int64_t device, at::Tensor word, at::Tensor mirror) {
   s.pair = {word.data_ptr<int>(), mirror.data_ptr<int>()};
 }
 
+[[noreturn]] void raise_status(DeviceStatus& s, int code) {
+  s.word.zero_();
+  s.mirror.zero_();
+  char msg[160];
+  std::snprintf(msg, sizeof(msg),
+                "flash_tt_attn: device status 0x%x (a bounded device-side wait ran out in an earlier call; its "
+                "outputs are incomplete)", code);
+  throw std::runtime_error(msg);
+}
+
 // An earlier launch's failed wait, seen through the mirror without touching the stream.
 DeviceStatus& status_of(c10::DeviceIndex device) {
   TORCH_CHECK(device >= 0 && device < kMaxDevices, "device index out of range");
   DeviceStatus& s = g_status[device];
   TORCH_CHECK(s.host != nullptr, "flash_tt_attn: no status word registered for this device");
   const int code = *s.host;
-  if (C10_UNLIKELY(code != 0)) {
-    s.word.zero_();
-    s.mirror.zero_();
-    char msg[160];
-    std::snprintf(msg, sizeof(msg),
-                  "flash_tt_attn: device status 0x%x (a bounded device-side wait ran out in an earlier call; its "
-                  "outputs are incomplete)", code);
-    throw std::runtime_error(msg);
-  }
+  if (C10_UNLIKELY(code != 0)) raise_status(s, code);
   return s;
+}
+
+// The same for the launches just made: waits for them.
+void check_status_now(const c10::Device& device) {
+  const c10::cuda::CUDAGuard guard(device);
+  DeviceStatus& s = status_of(device.index());
+  if (const int code = s.word.item<int>()) raise_status(s, code);
 }
 
 void ensure_status(const c10::Device& device) {
@@ -230,17 +239,19 @@ BackwardOut run_backward(const at::Tensor& q, const at::Tensor& k, const at::Ten
 
 struct Attention : public torch::autograd::Function<Attention> {
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
-                            const at::Tensor& bias, double sm_scale, const std::optional<at::Tensor>& key_mask) {
+                            const at::Tensor& bias, double sm_scale, const std::optional<at::Tensor>& key_mask, bool debug) {
     ForwardOut r = run_forward(q, k, v, bias, sm_scale, key_mask, true);
     ctx->save_for_backward({r.q, r.k, r.v, r.bias, r.o, r.saved});
     ctx->saved_data["sm_scale"] = sm_scale;
+    ctx->saved_data["debug"] = debug;
     return r.o;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
     TORCH_CHECK(grads[0].scalar_type() == s[0].scalar_type(), "the gradient of O must have O's dtype");
     BackwardOut r = run_backward(s[0], s[1], s[2], s[3], s[4], s[5], grads[0], ctx->saved_data["sm_scale"].toDouble(), true);
-    return {r.dq, r.dk, r.dv, r.dbias, at::Tensor(), at::Tensor()};
+    if (ctx->saved_data["debug"].toBool()) check_status_now(s[0].device());
+    return {r.dq, r.dk, r.dv, r.dbias, at::Tensor(), at::Tensor(), at::Tensor()};
   }
 };
 
@@ -271,8 +282,9 @@ void check_arguments(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
 
 bool has_tangent(const at::Tensor& t) { return t._fw_grad(/*level=*/0).defined(); }
 
+// `debug`: the backward pass waits for its launches and raises if one of them failed
 at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& bias,
-                     double sm_scale, const std::optional<at::Tensor>& key_mask) {
+                     double sm_scale, const std::optional<at::Tensor>& key_mask, bool debug) {
   check_arguments(q, k, v, bias, key_mask);
   py::gil_scoped_release no_gil;  // as torch's own operators do: an allocation or a full launch queue may wait
   const bool keep = at::GradMode::is_enabled() &&
@@ -281,7 +293,7 @@ at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
   // tangents and says so, where the bare pass would drop them.
   const bool dual = has_tangent(q) || has_tangent(k) || has_tangent(v) || has_tangent(bias);
   if (!keep && !dual) return run_forward(q, k, v, bias, sm_scale, key_mask, false).o;
-  return Attention::apply(q, k, v, bias, sm_scale, key_mask);
+  return Attention::apply(q, k, v, bias, sm_scale, key_mask, debug);
 }
 
 // For the Python autograd node of the sharded call (it puts a collective between the passes).

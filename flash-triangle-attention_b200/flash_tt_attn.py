@@ -147,6 +147,8 @@ class _attention(torch.autograd.Function):
                 check(_cabi.lib().fta_dbias_cast(db32.data_ptr(), db.data_ptr(), db32.numel(),
                                                  _cabi.FTA_BF16 if db.dtype == torch.bfloat16 else _cabi.FTA_FP16,
                                                  torch.cuda.current_stream().cuda_stream), "fta_dbias_cast")
+        if _DEBUG:
+            check_device_status(db.device)
         return dq, dk, dv, db, None, None, None
 
 
@@ -154,7 +156,7 @@ def _call(q, k, v, b_pw, sm_scale, group, key_mask):
     if group is not None:
         o = _attention.apply(q, k, v, b_pw, sm_scale, group, key_mask)
     else:
-        o = (_ext or _native()).attention(q, k, v, b_pw, float(sm_scale), key_mask)
+        o = (_ext or _native()).attention(q, k, v, b_pw, float(sm_scale), key_mask, _DEBUG)
     if _DEBUG:
         check_device_status(q.device)
     return o

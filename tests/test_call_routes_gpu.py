@@ -102,3 +102,34 @@ def test_other_threads_run_while_a_pass_waits_in_native_code(route):
     if longest < 0.1:
         pytest.skip(f"no launch had to wait (longest call {longest * 1e3:.1f} ms)")
     assert pause[0] < 0.5 * longest, (pause[0], longest)
+
+
+def _train():
+    q, k, v, b = _inputs()
+    q.requires_grad_()
+    return fta.attention(q, k, v, b, 0.2)
+
+
+def test_debug_mode_checks_the_backward_pass(monkeypatch):
+    """With FTA_DEBUG=1 a failure shows in the pass it happens in (the word is set by hand, as a wait that runs out
+    would)."""
+    monkeypatch.setattr(fta, "_DEBUG", True)
+    o = _train()
+    fta._status_of(o.device).word.fill_(0x1046)
+    with pytest.raises(RuntimeError, match="0x1046"):
+        o.sum().backward()
+    _train().sum().backward()
+    fta.check_device_status()
+
+
+def test_a_failure_in_a_backward_pass_raises_in_the_next_one_without_a_sync():
+    """The last kernel of a backward pass mirrors the word; the next backward pass looks at the mirror on the autograd
+    thread before it launches anything."""
+    first, second, third = _train(), _train(), _train()
+    fta._status_of(first.device).word.fill_(0x1047)
+    first.sum().backward()  # its last kernel mirrors the word
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="0x1047"):
+        second.sum().backward()
+    third.sum().backward()  # cleared when it was reported
+    fta.check_device_status()
