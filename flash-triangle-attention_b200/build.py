@@ -16,7 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libfta.so")
 SOURCES = ["api.cu", "fwd_sm100.cu", "bwd_sm100.cu", "stream_kernels.cu", "noalloc.cu"]
-HEADERS = ["tc05.cuh", "tmap.h", "fta_kernels.h", "native_api.h", os.path.join("..", "..", "include", "fta.h")]
+HEADERS = ["tc05.cuh", "tmap.h", "fta_kernels.h", "schedule.h", "native_api.h", os.path.join("..", "..", "include", "fta.h")]
 TORCH_EXT = os.path.join(HERE, "_fta_torch.so")
 TORCH_SOURCE = "torch_binding.cpp"
 NVCC_FLAGS = [

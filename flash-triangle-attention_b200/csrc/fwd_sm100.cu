@@ -28,6 +28,7 @@
 // owns the query row; the O accumulator is rescaled whenever the row max grew, by the same
 // thread, before P is handed to the PV MMA.
 #include "fta_kernels.h"
+#include "schedule.h"
 #include "tc05.cuh"
 
 namespace fta {
@@ -545,36 +546,9 @@ int launch_fwd_t(const FwdArgs& a, cudaStream_t stream) {
   p.scale = a.sm_scale;
   p.stat_pitch = (a.L2 + 127) / 128 * 128;
   p.stat_stride = static_cast<long long>(a.B) * a.H * a.L1 * p.stat_pitch;
-  // Row groups are dealt round-robin to grid.y CTAs per (query block, head). Pick the smallest
-  // grid.y whose schedule (waves of one CTA per SM, the longest CTA setting the pace) is within
-  // 3 % of the best: few long-lived CTAs amortise their start-up and keep the pipeline full
-  // across row groups.
-  const int ngroups = (a.L1 + kRows - 1) / kRows;
   const long long per = static_cast<long long>((a.L2 + 127) / 128) * a.B * a.H;
-  const int sms = num_sms();
-  int best_gy = 1;
-  {
-    double best = 0.0;
-    const int gy_max = ngroups < 96 ? ngroups : 96;  // beyond that the last wave is a small part of any schedule
-    // first pass: best efficiency; second: smallest gy close to it
-    for (int pass = 0; pass < 2; ++pass) {
-      for (int gy = 1; gy <= gy_max; ++gy) {
-        const long long ctas = per * gy;
-        const long long waves = (ctas + sms - 1) / sms;
-        const int longest = (ngroups + gy - 1) / gy;
-        // fixed cost per CTA of about a third of a row group
-        const double eff = static_cast<double>(per) * ngroups /
-                           (static_cast<double>(waves) * sms * (longest + 0.35));
-        if (pass == 0) {
-          if (eff > best) best = eff;
-        } else if (eff >= 0.97 * best) {
-          best_gy = gy;
-          break;
-        }
-      }
-    }
-  }
-  dim3 grid((a.L2 + 127) / 128, best_gy, a.B * a.H);
+  const int grid_y = fwd_grid_rows((a.L1 + kRows - 1) / kRows, per, num_sms());
+  dim3 grid((a.L2 + 127) / 128, grid_y, a.B * a.H);
   return static_cast<int>(launch_overlapped(kern, grid, 384, C::SMEM_BYTES, stream, a.tmQ, a.tmK, a.tmV, a.tmBias, p));
 }
 
