@@ -11,7 +11,10 @@ namespace {
 thread_local int g_last_cuda_error = 0;
 thread_local cudaEvent_t g_prof_start = nullptr, g_prof_stop = nullptr;
 
+// Every failed runtime call ends here. The runtime keeps its error until somebody asks, and the launches ask to learn
+// how they went: what is reported here must not be found again by the next, healthy one.
 int cuda_fail(cudaError_t e) {
+  cudaGetLastError();
   g_last_cuda_error = static_cast<int>(e);
   return FTA_ERR_CUDA;
 }

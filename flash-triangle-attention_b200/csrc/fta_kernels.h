@@ -10,11 +10,11 @@
 namespace fta {
 
 // Records `cuda_error` (a cudaError_t) as the calling thread's last CUDA error, the value
-// fta_last_cuda_error() reports; returns FTA_ERR_CUDA.
+// fta_last_cuda_error() reports, and clears the runtime's own record of it; returns FTA_ERR_CUDA.
 int record_cuda_error(int cuda_error);
 
 // Every launch_* function below returns cudaSuccess (0) or the cudaError_t of the call that failed
-// (the launch itself or an attribute call before it); it leaves no sticky error behind.
+// (the launch itself or an attribute call before it), which the caller hands to record_cuda_error.
 
 // cudaFuncAttributeMaxDynamicSharedMemorySize is a property of a kernel ON ONE DEVICE: a process
 // that drives several GPUs has to set it once per device. One flag per device ordinal; two threads

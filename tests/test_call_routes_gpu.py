@@ -133,3 +133,30 @@ def test_a_failure_in_a_backward_pass_raises_in_the_next_one_without_a_sync():
         second.sum().backward()
     third.sum().backward()  # cleared when it was reported
     fta.check_device_status()
+
+
+def test_a_refused_call_does_not_fail_the_next_one():
+    """The runtime refuses to wait for a stream that is being captured, on the host. That error belongs to that call
+    alone: launches learn how they went from the runtime's last error."""
+    import ctypes
+    import _cabi
+    L = _cabi.lib()
+    rt = ctypes.CDLL("libcudart.so.12")  # torch's; a stream means the same to every runtime of the process
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    x = torch.ones(64, device="cuda")
+    y = torch.zeros(64, device="cuda", dtype=torch.bfloat16)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    handle, code, graph = ctypes.c_void_p(side.cuda_stream), ctypes.c_int32(0), ctypes.c_void_p()
+    relaxed = 2
+    assert rt.cudaStreamBeginCapture(handle, relaxed) == 0
+    try:
+        assert L.fta_read_status(status.data_ptr(), ctypes.byref(code), side.cuda_stream) == -9  # FTA_ERR_CUDA
+        refused = L.fta_last_cuda_error()
+    finally:
+        rt.cudaStreamEndCapture(handle, ctypes.byref(graph))  # says that the capture came to nothing
+        rt.cudaGetLastError()
+    assert refused != 0
+    st = torch.cuda.current_stream().cuda_stream
+    assert L.fta_dbias_cast(x.data_ptr(), y.data_ptr(), 64, _cabi.FTA_BF16, st) == 0
+    assert float(y.sum()) == 64.0 and L.fta_last_cuda_error() == refused
