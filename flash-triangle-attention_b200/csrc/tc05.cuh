@@ -93,7 +93,13 @@ __device__ __forceinline__ uint32_t mbar_try_wait_hint(uint32_t bar, uint32_t pa
 struct WaitCtx {
   uint32_t abort_addr;  // shared-memory address of the CTA's abort word
   int* status;          // global memory, one per launch
-  unsigned long long limit_ns = 1000000000ull;  // a wait gives up after this long (about a second)
+  unsigned long long limit_ns = 1000000000ull;  // a wait gives up after this long (about a second); at most kMaxWaitNs
+
+  // Counted in SM clock cycles, two to the nanosecond, by a 32-bit clock: a longer limit would wrap to a short one.
+  static constexpr unsigned long long kMaxWaitNs = 2000000000ull;
+  __device__ __forceinline__ uint32_t limit_cycles() const {
+    return static_cast<uint32_t>(2ull * (limit_ns < kMaxWaitNs ? limit_ns : kMaxWaitNs));
+  }
 };
 
 
@@ -122,7 +128,7 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
 // caller must then skip to the tear-down, and the roles that wait for it run out in turn.
 // Kept to a dozen instructions: a kernel inlines this at some forty places, and what lies between the instructions
 // of its loops is fetched with them (measured: a straight loop body beyond 32 KB runs at a third of its issue
-// rate). The limit is counted in SM clock cycles, two to the nanosecond.
+// rate).
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const WaitCtx& w, int site) {
   // one poll and one vote; try_wait suspends the thread for a short time bounded by the hardware and the hint
   auto poll = [&] {
@@ -142,7 +148,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, co
   const uint32_t t0 = sm_clock();
 #pragma unroll 1
   while (!poll()) {
-    if (!__any_sync(0xffffffffu, sm_clock() - t0 > static_cast<uint32_t>(2u * w.limit_ns))) continue;
+    if (!__any_sync(0xffffffffu, sm_clock() - t0 > w.limit_cycles())) continue;
     st_shared_volatile_u32(w.abort_addr, 1u);
     atomicCAS(w.status, kStatusOk, kStatusWaitTimeout | site);
     return false;

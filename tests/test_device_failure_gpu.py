@@ -72,6 +72,18 @@ def test_bounded_wait_runs_out_records_status_and_returns(probe):
     assert torch.isfinite(q.grad).all()
 
 
+def test_a_long_wait_limit_is_cut_not_wrapped(probe):
+    """The limit is counted by a 32-bit clock: 2.2 s is 4.4e9 cycles, which wrapped to a tenth of a second's worth. It
+    is cut to two seconds."""
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    waited = torch.zeros(1, dtype=torch.int64, device="cuda")
+    assert probe.wait_probe_launch(status.data_ptr(), 0, 2_200_000_000, waited.data_ptr(),
+                                   torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0x1000 | 0x7
+    assert 1_500_000_000 <= int(waited.item()) <= 6_000_000_000  # 4e9 cycles, whatever the clock does
+
+
 def test_status_word_of_an_earlier_call_surfaces_without_a_sync():
     """The module mirrors its status word to pinned host memory after every call and looks at the
     mirror before the next launch: a recorded failure raises at the next call (here the word is
