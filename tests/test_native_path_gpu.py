@@ -108,3 +108,54 @@ def test_streamed_call_with_blocks_that_need_more_scratch_than_the_largest(B, H,
     assert float((out["dq"].float() - leaves[0].grad.cpu().float()).abs().max()) <= float(out["dq"].float().abs().max()) * 2.0 ** -8
     ref = fta.last_dbias_f32()
     assert float((db32 - ref).abs().max()) <= 1e-4 * float(ref.abs().max()) + 1e-5
+
+
+@pytest.mark.parametrize("L1,L2,D", [(3, 104, 32), (2, 128, 64), (4, 200, 32), (2, 264, 64)])
+@pytest.mark.parametrize("layout", ["rows_exchanged", "padded"])
+def test_outputs_of_any_strides_and_nothing_beside_them(L1, L2, D, layout):
+    """Through the C ABI the caller lays out O and the gradients. With one key block dQ, and always dK and dV, leave
+    through tensor maps made from those strides; the elements between and behind the rows keep what they held."""
+    import _cabi
+    from _cabi import FtaProblem, check, t4, t5
+    B, H, dt = 2, 2, torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(L2)
+    q, k, v, do = (torch.randn(B, H, L1, L2, D, device="cuda", dtype=dt, generator=g) for _ in range(4))
+    b = torch.randn(B, H, L2, L2, device="cuda", dtype=dt, generator=g)
+    leaves = [x.clone().requires_grad_() for x in (q, k, v, b)]
+    want_o = fta.attention(*leaves, 0.2)
+    want_o.backward(do)
+
+    def out():
+        if layout == "rows_exchanged":
+            whole = torch.full((B, L2 + 1, H, L1 + 1, D + 8), 77.0, device="cuda", dtype=dt)
+            return whole, whole[:, :L2, :, :L1, :D].permute(0, 2, 3, 1, 4)
+        whole = torch.full((B, H, L1 + 1, L2 + 3, D + 8), 77.0, device="cuda", dtype=dt)
+        return whole, whole[:, :, :L1, :L2, :D]
+
+    outs = {n: out() for n in ("o", "dq", "dk", "dv")}
+    view = {n: t5(x[1]) for n, x in outs.items()}
+    L, prob, st = _cabi.lib(), FtaProblem(B, H, L1, L2, D, _cabi.FTA_BF16), torch.cuda.current_stream().cuda_stream
+    pitch = (L2 + 127) // 128 * 128
+    f32 = lambda *s: torch.empty(s, device="cuda")
+    lse, delta, db32, status = f32(3, B, H, L1, pitch), f32(B, H, L1, pitch), f32(B, H, L2, L2), torch.zeros(1, dtype=torch.int32, device="cuda")
+    bias = b
+    if pitch != L2:
+        bias = torch.empty(B, H, pitch, pitch, device="cuda", dtype=dt)
+        check(L.fta_mask_bias(prob, t4(b), None, bias.data_ptr(), st), "fta_mask_bias")
+    check(L.fta_forward(prob, t5(q), t5(k), t5(v), t4(bias), 0.2, view["o"], None, lse.data_ptr(), status.data_ptr(), st), "fta_forward")
+    # without the rounding residual of O, which attention() adds to delta: dQ and dK agree within bf16
+    check(L.fta_bwd_preprocess(prob, view["o"], None, t5(do), delta.data_ptr(), st), "fta_bwd_preprocess")
+    ws = torch.empty(L.fta_bwd_workspace_bytes(prob), dtype=torch.uint8, device="cuda")
+    check(L.fta_backward(prob, t5(q), t5(k), t5(v), t4(bias), t5(do), lse.data_ptr(), delta.data_ptr(), 0.2, view["dq"], view["dk"],
+                         view["dv"], db32.data_ptr(), None, ws.data_ptr(), ws.numel(), status.data_ptr(), st), "fta_backward")
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    want = {"o": want_o.detach(), "dq": leaves[0].grad, "dk": leaves[1].grad, "dv": leaves[2].grad}
+    for n, (whole, x) in outs.items():
+        a, w = x.float().cpu().numpy(), want[n].float().cpu().numpy()
+        assert npo.rel_l2(a, w) <= 1e-2, (n, npo.rel_l2(a, w))
+        if n in ("o", "dv"):  # no delta in these
+            assert np.array_equal(a, w), n
+        untouched = torch.ones_like(whole, dtype=torch.bool)
+        (untouched[:, :L2, :, :L1, :D] if layout == "rows_exchanged" else untouched[:, :, :L1, :L2, :D]).fill_(False)
+        assert bool((whole[untouched] == 77.0).all()), n
