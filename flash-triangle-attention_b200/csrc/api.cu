@@ -171,7 +171,7 @@ int backward(const FtaProblem* prob, int nplanes, const fta::PreArgs* pre, const
       (rc = check_t5(dq)) || (rc = check_t5(dk)) || (rc = check_t5(dv)) || (rc = check_t4(bias)))
     return rc;
   if (!lse || !delta || !dbias_f32 || !status.word || !workspace) return FTA_ERR_NULL;
-  // the kernel fetches the statistics with 512-byte bulk copies and the epilogue writes dBias with
+  // the kernel fetches the statistics with 256-byte bulk copies and the epilogue writes dBias with
   // 16-byte stores
   if (!aligned16(lse) || !aligned16(delta) || !aligned16(dbias_f32) || !aligned16(dbias_cast)) return FTA_ERR_ALIGN;
   if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0 || have_bytes < workspace_bytes(prob, nplanes))
@@ -214,7 +214,6 @@ int backward(const FtaProblem* prob, int nplanes, const fta::PreArgs* pre, const
   }
   a.lse = lse;
   a.delta = delta;
-  a.dq32 = dq32;
   a.status = status.word;
   a.nplanes = nplanes;
   a.B = prob->B;

@@ -109,7 +109,6 @@ struct BwdCfg {
 struct BwdParams {
   const float* lse;  // three planes: -max (natural-log units), -log2(sum), c (see the forward kernel)
   const float* delta;
-  float* dq32;
   int* status;
   int H, L1, L2, NP, BH;
   int stat_pitch;  // row pitch of lse / delta: L2 rounded up to 128
@@ -734,7 +733,6 @@ int launch_bwd_t(const BwdArgs& a, int NP, cudaStream_t stream) {
   BwdParams p;
   p.lse = a.lse;
   p.delta = a.delta;
-  p.dq32 = a.dq32;
   p.status = a.status;
   p.H = a.H;
   p.L1 = a.L1;

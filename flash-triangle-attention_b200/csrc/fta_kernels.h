@@ -89,16 +89,16 @@ struct FwdArgs {
   float sm_scale;
 };
 int launch_fwd(const FwdArgs& a, cudaStream_t stream);
-int fwd_rows_per_cta(int D);
 
 struct BwdArgs {
   CUtensorMap tmQ, tmK, tmV, tmDO, tmBiasT;  // tmBiasT: over the key-major copy of the bias
-  CUtensorMap tmDQ;    // dq32 as a 3-D float32 tensor (B*H*L1, L2, D), box 128 queries x 32 columns, 128 B swizzle
+  CUtensorMap tmDQ;    // the float32 dQ accumulator as (B*H*L1, L2, D), box 32 queries x 16 columns, 64 B swizzle: zeroed
+                       // before, receives the sum over the key blocks of dS K (not used for L2 <= 128)
   CUtensorMap tmDK, tmDV, tmDQ16;  // the 16-bit outputs, boxes of 32 columns x 32 rows, 64 B swizzle (tmDQ16: L2 <= 128)
-  CUtensorMap tmPlane; // the partial dBias planes as (nplanes*B*H, L2 keys, L2 queries) float32, same box
-  const float* lse;    // (3,B,H,L1,L2): -max, -log2(sum), combined (NaN where inexact)
-  const float* delta;  // (B,H,L1,L2)
-  float* dq32;         // (B,H,L1,L2,D) float32, zeroed; receives sum over key blocks of dS K (not used for L2 <= 128)
+  CUtensorMap tmPlane; // the partial dBias planes as (nplanes*B*H, L2 keys, L2 queries) float32, box 128 keys x
+                       // 32 queries, 128 B swizzle
+  const float* lse;    // (3,B,H,L1,L2p), L2p = L2 rounded up to 128: -max, -log2(sum), combined (NaN where inexact)
+  const float* delta;  // (B,H,L1,L2p)
   int* status;
   int B, H, L1, L2, D;
   int nplanes;  // bwd_num_planes()
@@ -135,9 +135,10 @@ int launch_mask_bias(const void* bias, const long long sb[4], const uint8_t* key
 int launch_bwd_prologue(const void* bias, const long long sb[4], void* bias_t, int B, int H, int L2, float* dq32,
                         long long dq_elems, const PreArgs* pre, cudaStream_t stream);
 
-// Backward epilogue, one launch: dq[row, d] = (dtype)(scale * dq32[row, d]) and, for the KEY-MAJOR
-// (dq32 == nullptr: dq has been written already) planes the backward kernel writes, (nplanes, B*H, key, query) with rows of L2 rounded up to 8 elements:
-// dbias_f32[bh][query][key] = sum_p planes[p][bh][key][query] in plane order, optional rounded copy
+// Backward epilogue, one launch: dq[row, d] = (dtype)(scale * dq32[row, d]) (dq32 == nullptr: dq has been written
+// already) and dbias_f32[bh][query][key] = sum_p planes[p][bh][key][query] in plane order, with an optional rounded
+// copy, for the key-major planes that the backward kernel writes: (nplanes, B*H, key, query), rows of L2 rounded up to 8
+// elements
 int launch_bwd_epilogue(const float* dq32, void* dq, const long long sdq[4], int B, int H, int L1, int L2, int D,
                         float scale, const float* planes, int nplanes, float* dbias_f32, void* dbias_cast, bool bf16,
                         Status status, cudaStream_t stream);

@@ -566,6 +566,4 @@ int launch_fwd(const FwdArgs& a, cudaStream_t stream) {
   return a.bf16 ? launch_fwd_t<64, true, 2>(a, stream) : launch_fwd_t<64, false, 2>(a, stream);
 }
 
-int fwd_rows_per_cta(int D) { return D == 32 ? FwdCfg<32>::G : FwdCfg<64>::G; }
-
 }  // namespace fta

@@ -3,8 +3,10 @@
 // UMMA shared-memory / instruction descriptors, tcgen05.mma / ld / st wrappers.
 //
 // Every wait in this file is bounded: a wait that runs out records a code in a status
-// word and raises a CTA-wide abort flag so that all roles fall through to the tear-down
-// (free tensor memory, return). Nothing here traps or spins forever.
+// word and raises a CTA-wide flag, and its role falls through to the tear-down; the roles
+// that wait for that one run out in turn, each by its own limit. The tear-down (leave copies in
+// flight time to land where the flag is set, free tensor memory, return) is reached by all. Nothing here
+// traps or spins forever.
 #pragma once
 
 #include <cuda.h>
@@ -59,37 +61,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok;
-}
-
-// Same with a suspend-time hint: the hardware may park the thread for up to `hint_ns` and
-// wakes it when the phase completes, so a waiting warp does not burn issue slots polling.
-__device__ __forceinline__ uint32_t mbar_try_wait_hint(uint32_t bar, uint32_t parity, uint32_t hint_ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(hint_ns)
-      : "memory");
-  return ok;
-}
-
-// Shared abort flag + global status word, carried by every role.
+// The CTA's abort word (raised by a wait that ran out, looked at by the tear-down) and the global status word, carried
+// by every role.
 struct WaitCtx {
   uint32_t abort_addr;  // shared-memory address of the CTA's abort word
   int* status;          // global memory, one per launch
@@ -102,12 +75,6 @@ struct WaitCtx {
   }
 };
 
-
-__device__ __forceinline__ uint32_t ld_shared_volatile_u32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-  return v;
-}
 __device__ __forceinline__ void st_shared_volatile_u32(uint32_t addr, uint32_t v) {
   asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
@@ -204,21 +171,10 @@ __device__ __forceinline__ void tc_fence_after_sync() {
 }
 
 // ----------------------------------------------------------------------------------
-// TMA tile loads (no multicast anywhere)
+// TMA tiles (no multicast anywhere; coordinates innermost first)
 // ----------------------------------------------------------------------------------
-// shared -> global tile transfers (bulk async-group completion): add into / overwrite a 2-D tile
-__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* tmap, uint32_t src, int c0, int c1) {
-  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1)
-               : "memory");
-}
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* tmap, uint32_t src, int c0, int c1) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1)
-               : "memory");
-}
-// the same for 3-D tiles (coordinates innermost first); parts of a tile that lie beyond the tensor's
-// extents are clipped
+// shared -> global tile transfers (bulk async-group completion): add into / overwrite a tile; the parts of it that
+// lie beyond the tensor's extents are clipped
 __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* tmap, uint32_t src, int c0, int c1, int c2) {
   asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
                ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1), "r"(c2)
@@ -263,15 +219,6 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
 }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tmap, uint32_t bar,
-                                            int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
 }
 
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* tmap, uint32_t bar,
@@ -326,21 +273,6 @@ __device__ __forceinline__ void tma_load_4d_hint(uint32_t dst, const CUtensorMap
       "r"(c3), "l"(pol)
       : "memory");
 }
-__device__ __forceinline__ void tma_reduce_add_2d_hint(const CUtensorMap* tmap, uint32_t src, int c0, int c1,
-                                                       uint64_t pol) {
-  asm volatile(
-      "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group.L2::cache_hint [%0, {%2, %3}], [%1], %4;"
-      ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1), "l"(pol)
-      : "memory");
-}
-__device__ __forceinline__ void tma_store_2d_hint(const CUtensorMap* tmap, uint32_t src, int c0, int c1,
-                                                  uint64_t pol) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group.L2::cache_hint [%0, {%2, %3}], [%1], %4;"
-      ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1), "l"(pol)
-      : "memory");
-}
-
 // ----------------------------------------------------------------------------------
 // tensor memory (TMEM) allocation: executed by one full warp
 // ----------------------------------------------------------------------------------
@@ -362,7 +294,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 // UMMA descriptors
 // ----------------------------------------------------------------------------------
 // Swizzle modes of the shared-memory matrix descriptor (bits 61..63).
-enum : uint64_t { kSwzNone = 0, kSwz128 = 2, kSwz64 = 4, kSwz32 = 6 };
+enum : uint64_t { kSwz128 = 2, kSwz64 = 4 };
 
 // Shared-memory matrix descriptor. `lbo`/`sbo` are byte offsets (multiples of 16).
 //   K-major operand, swizzled:  sbo = bytes between 8-row groups, lbo unused.
