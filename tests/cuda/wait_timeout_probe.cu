@@ -1,5 +1,5 @@
 // Test-only kernel (never part of libfta.so): exercises the bounded mbarrier wait of the product
-// kernels (csrc/tc05.cuh: mbar_wait / mbar_wait_warp) when nobody arrives. The wait is given a
+// kernels (csrc/tc05.cuh: mbar_wait_warp) when nobody arrives. The wait is given a
 // limit of a few milliseconds; it must run out, record 0x1000 | site in the status word, raise
 // the CTA's abort flag, let every role reach the tear-down (tensor memory freed) and return - no
 // trap, no hang - so that the context stays usable for the next launch.

@@ -2,7 +2,7 @@
 
 Nothing here faults, traps or hangs a GPU: the failure is a wait on a barrier that nobody arrives
 at, and the wait gives up by itself after a few milliseconds (tests/cuda/wait_timeout_probe.cu uses
-the product's own ``mbar_wait`` from csrc/tc05.cuh with a small limit).
+the product's own ``mbar_wait_warp`` from csrc/tc05.cuh with a small limit).
 """
 import ctypes
 import os
@@ -85,8 +85,8 @@ def test_a_long_wait_limit_is_cut_not_wrapped(probe):
 
 
 def test_status_word_of_an_earlier_call_surfaces_without_a_sync():
-    """The module mirrors its status word to pinned host memory after every call and looks at the
-    mirror before the next launch: a recorded failure raises at the next call (here the word is
+    """The forward kernel mirrors a word that is not zero in pinned host memory as it ends, and the module looks
+    at the mirror before the next launch: a recorded failure raises at the next call (here the word is
     set by hand, as a kernel whose wait ran out would)."""
     dev = torch.device("cuda", torch.cuda.current_device())
     q = torch.randn(1, 1, 2, 128, 32, device="cuda", dtype=torch.float16)
