@@ -35,10 +35,11 @@
 // gets out 32 bytes per cycle of stores and 25 of float32 reductions (30 and 24 with all SMs at it): at D = 32 a tile's
 // 16 KB of dQ and third of 64 KB of dBias need 1 560 cycles, at D = 64 32 KB and 64 KB need 4 100.
 //
-// Measured (main kernel, B1 H4 L1 96 L2 768 D32 bf16): 256 -> 221 us against four quarter-tile warpgroups moving in
-// step through two phases per tile, each phase with its own hand-over. A tile takes about 3 500 cycles, of which a
+// Measured (main kernel, B1 H4 L1 96 L2 768 D32 bf16): 256 -> 197 us against four quarter-tile warpgroups moving in
+// step through two phases per tile, each phase with its own hand-over. A tile takes about 3 770 cycles, of which a
 // half's pass is 1 500 (512 are its exponentials; two warps per scheduler do not hide the latencies of the
-// chain), hand-over to hand-over 700, and a third of a flush 500.
+// chain), hand-over to hand-over 700, and a third of a flush 500. At D = 64 it takes 7 200 (L2 512) to 10 800 (L2 2048, where
+// the planes pass the L2 cache).
 // Tried: the four quarters with a hand-over each (768 threads, 96 registers): the issuer, at a good 1 000 cycles per
 // turn, became the bound (3.18 ms at L768 against 2.71); 16 queries per TMEM load instead of 8: equal.
 //
