@@ -398,54 +398,58 @@ def attention_fwd_bwd_streamed(host, sm_scale, out, block_rows=96, device=None, 
         ev_comp = [torch.cuda.Event() for _ in range(NSLOT)]
         ev_out = [torch.cuda.Event() for _ in range(NSLOT)]
         bias = torch.empty(b_h.shape, dtype=b_h.dtype, device=dev)  # from the current stream's pool
-        s_in.wait_stream(cur)
-        with torch.cuda.stream(s_in):
-            bias.copy_(b_h, non_blocking=True)
-        cur.wait_stream(s_in)
-        bias_k = bias
-        if L2p != L2:
-            bias_k = mk(B, H, L2p, L2p)
-            check(L.fta_mask_bias(FtaProblem(B, H, 1, L2, D, dtype_code), t4(bias), None, bias_k.data_ptr(), cur.cuda_stream),
-                  "fta_mask_bias")
-        bias4 = t4(bias_k)
-        db32 = torch.zeros((B, H, L2, L2), dtype=torch.float32, device=dev)
-        db_blk = torch.empty_like(db32)
-        resid = q_h.dtype == torch.bfloat16 and _SAVE_O_RESIDUAL
-        r0 = 0
-        for blk, n in enumerate(sizes):
-            slot = blk % NSLOT
-            sl = slots[slot]
-            if blk >= NSLOT:
-                s_in.wait_event(ev_comp[slot])  # the kernels of block blk - NSLOT have read this slot's inputs
-                cur.wait_event(ev_out[slot])    # ... and its results are on their way out of the output buffers
-            for name in names_in:
-                _copy_rows(L, sl[name], 0, host[name], r0, n, s_in.cuda_stream)
-            ev_in[slot].record(s_in)
-            cur.wait_event(ev_in[slot])
-            prob = FtaProblem(B, H, n, L2, D, dtype_code)
-            v5 = {k: t5(sl[k][:, :, :n]) for k in names_in + names_out}
-            ores_ptr = sl["ores"].data_ptr() if resid else None
-            # the residual buffer is addressed with the strides of `o` (the slot's full block)
-            check(L.fta_forward(prob, v5["q"], v5["k"], v5["v"], bias4, float(sm_scale), v5["o"], ores_ptr,
-                                sl["lse"].data_ptr(), st.word.data_ptr(), cur.cuda_stream), "fta_forward")
-            check(L.fta_bwd_preprocess(prob, v5["o"], ores_ptr, v5["do"], sl["delta"].data_ptr(), cur.cuda_stream),
-                  "fta_bwd_preprocess")
-            check(L.fta_backward(prob, v5["q"], v5["k"], v5["v"], bias4, v5["do"], sl["lse"].data_ptr(),
-                                 sl["delta"].data_ptr(), float(sm_scale), v5["dq"], v5["dk"], v5["dv"],
-                                 db_blk.data_ptr(), None, ws.data_ptr(), ws_bytes, st.word.data_ptr(), cur.cuda_stream),
-                  "fta_backward")
-            db32 += db_blk
-            ev_comp[slot].record(cur)
-            s_out.wait_event(ev_comp[slot])
-            for name in names_out:
-                _copy_rows(L, out[name], r0, sl[name], 0, n, s_out.cuda_stream)
-            ev_out[slot].record(s_out)
-            r0 += n
-        if group is not None:
-            torch.distributed.all_reduce(db32, op=torch.distributed.ReduceOp.SUM, group=group)
-        out["dbias"].copy_(db32.to(b_h.dtype), non_blocking=True)
-        _native().set_last_dbias_f32(db32)
-        st.publish()
-        cur.wait_stream(s_out)
-        torch.cuda.synchronize(dev)
+        try:
+            s_in.wait_stream(cur)
+            with torch.cuda.stream(s_in):
+                bias.copy_(b_h, non_blocking=True)
+            cur.wait_stream(s_in)
+            bias_k = bias
+            if L2p != L2:
+                bias_k = mk(B, H, L2p, L2p)
+                check(L.fta_mask_bias(FtaProblem(B, H, 1, L2, D, dtype_code), t4(bias), None, bias_k.data_ptr(), cur.cuda_stream),
+                      "fta_mask_bias")
+            bias4 = t4(bias_k)
+            db32 = torch.zeros((B, H, L2, L2), dtype=torch.float32, device=dev)
+            db_blk = torch.empty_like(db32)
+            resid = q_h.dtype == torch.bfloat16 and _SAVE_O_RESIDUAL
+            r0 = 0
+            for blk, n in enumerate(sizes):
+                slot = blk % NSLOT
+                sl = slots[slot]
+                if blk >= NSLOT:
+                    s_in.wait_event(ev_comp[slot])  # the kernels of block blk - NSLOT have read this slot's inputs
+                    cur.wait_event(ev_out[slot])    # ... and its results are on their way out of the output buffers
+                for name in names_in:
+                    _copy_rows(L, sl[name], 0, host[name], r0, n, s_in.cuda_stream)
+                ev_in[slot].record(s_in)
+                cur.wait_event(ev_in[slot])
+                prob = FtaProblem(B, H, n, L2, D, dtype_code)
+                v5 = {k: t5(sl[k][:, :, :n]) for k in names_in + names_out}
+                ores_ptr = sl["ores"].data_ptr() if resid else None
+                # the residual buffer is addressed with the strides of `o` (the slot's full block)
+                check(L.fta_forward(prob, v5["q"], v5["k"], v5["v"], bias4, float(sm_scale), v5["o"], ores_ptr,
+                                    sl["lse"].data_ptr(), st.word.data_ptr(), cur.cuda_stream), "fta_forward")
+                check(L.fta_bwd_preprocess(prob, v5["o"], ores_ptr, v5["do"], sl["delta"].data_ptr(), cur.cuda_stream),
+                      "fta_bwd_preprocess")
+                check(L.fta_backward(prob, v5["q"], v5["k"], v5["v"], bias4, v5["do"], sl["lse"].data_ptr(),
+                                     sl["delta"].data_ptr(), float(sm_scale), v5["dq"], v5["dk"], v5["dv"],
+                                     db_blk.data_ptr(), None, ws.data_ptr(), ws_bytes, st.word.data_ptr(), cur.cuda_stream),
+                      "fta_backward")
+                db32 += db_blk
+                ev_comp[slot].record(cur)
+                s_out.wait_event(ev_comp[slot])
+                for name in names_out:
+                    _copy_rows(L, out[name], r0, sl[name], 0, n, s_out.cuda_stream)
+                ev_out[slot].record(s_out)
+                r0 += n
+            if group is not None:
+                torch.distributed.all_reduce(db32, op=torch.distributed.ReduceOp.SUM, group=group)
+            out["dbias"].copy_(db32.to(b_h.dtype), non_blocking=True)
+            _native().set_last_dbias_f32(db32)
+            st.publish()
+            cur.wait_stream(s_out)
+            torch.cuda.synchronize(dev)
+        except BaseException:
+            torch.cuda.synchronize(dev)  # copies in flight use buffers that end with this call
+            raise
     check_device_status(dev)

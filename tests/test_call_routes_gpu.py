@@ -160,3 +160,22 @@ def test_a_refused_call_does_not_fail_the_next_one():
     st = torch.cuda.current_stream().cuda_stream
     assert L.fta_dbias_cast(x.data_ptr(), y.data_ptr(), 64, _cabi.FTA_BF16, st) == 0
     assert float(y.sum()) == 64.0 and L.fta_last_cuda_error() == refused
+
+
+def test_a_streamed_call_that_raises_leaves_no_copy_in_flight(monkeypatch):
+    """The device buffers of the call die with it: copies on its own streams must not outlive them, and the caller's
+    host tensors are the caller's again."""
+    host = {n: torch.randn(1, 4, 288, 512, 64).bfloat16().pin_memory() for n in ("q", "k", "v", "do")}
+    host["bias"] = torch.randn(1, 4, 512, 512).bfloat16().pin_memory()
+    out = {n: torch.empty_like(host["q"]).pin_memory() for n in ("o", "dq", "dk", "dv")}
+    out["dbias"] = torch.empty_like(host["bias"]).pin_memory()
+    fta.attention_fwd_bwd_streamed(host, 0.2, out)
+    want = out["o"].clone()
+    with monkeypatch.context() as m:
+        m.setattr(fta, "_blocks_workspace_bytes", lambda *a: 256)  # refused on the host by the first fta_backward
+        with pytest.raises(fta._cabi.FtaError):
+            fta.attention_fwd_bwd_streamed(host, 0.2, out)
+        streams = fta._copy_streams["cuda", torch.cuda.current_device()]
+        assert all(s.query() for s in (*streams, torch.cuda.current_stream()))
+    fta.attention_fwd_bwd_streamed(host, 0.2, out)
+    assert torch.equal(out["o"], want)
