@@ -243,14 +243,14 @@ struct Attention : public torch::autograd::Function<Attention> {
     ForwardOut r = run_forward(q, k, v, bias, sm_scale, key_mask, true);
     ctx->save_for_backward({r.q, r.k, r.v, r.bias, r.o, r.saved});
     ctx->saved_data["sm_scale"] = sm_scale;
-    ctx->saved_data["debug"] = debug;
+    if (debug) ctx->saved_data["debug"] = true;
     return r.o;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
     TORCH_CHECK(grads[0].scalar_type() == s[0].scalar_type(), "the gradient of O must have O's dtype");
     BackwardOut r = run_backward(s[0], s[1], s[2], s[3], s[4], s[5], grads[0], ctx->saved_data["sm_scale"].toDouble(), true);
-    if (ctx->saved_data["debug"].toBool()) check_status_now(s[0].device());
+    if (C10_UNLIKELY(ctx->saved_data.count("debug") != 0)) check_status_now(s[0].device());
     return {r.dq, r.dk, r.dv, r.dbias, at::Tensor(), at::Tensor(), at::Tensor()};
   }
 };
