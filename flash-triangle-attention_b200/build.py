@@ -15,7 +15,7 @@ import sysconfig
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libfta.so")
-SOURCES = ["api.cu", "fwd_sm100.cu", "bwd_sm100.cu", "stream_kernels.cu", "noalloc.cu"]
+SOURCES = ["api.cu", "fwd_sm100.cu", "fwd_quad_sm100.cu", "bwd_sm100.cu", "stream_kernels.cu", "noalloc.cu"]
 HEADERS = ["tc05.cuh", "tmap.h", "fta_kernels.h", "schedule.h", "native_api.h", os.path.join("..", "..", "include", "fta.h")]
 TORCH_EXT = os.path.join(HERE, "_fta_torch.so")
 TORCH_SOURCE = "torch_binding.cpp"

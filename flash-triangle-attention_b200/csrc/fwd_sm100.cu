@@ -1,5 +1,6 @@
 // Forward triangle attention for sm_100a: O = softmax(sm_scale * q k^T + bias) v and the
 // softmax statistics (row max and log2 of the row sum), the work of the reference's `_attn_fwd` (flash_tt_attn.py:128-264).
+// For D = 64 with more than a few key blocks and for small problems; the others go to fwd_quad_sm100.cu (see launch_fwd).
 //
 // One CTA owns a 128-query block `jb` of one (b,h) and walks a residue class of the groups of G
 // consecutive L1 rows back to back (loads and MMAs of the next group start while the softmax
@@ -39,7 +40,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 template <int kD>
 struct FwdCfg {
-  static constexpr int G = (kD == 32) ? 4 : 2;       // rows per CTA (even)
+  static constexpr int G = 2;                        // rows per group, one per softmax warpgroup
   static constexpr int NSTAGE = (kD == 32) ? 6 : 4;  // K/V ring depth
   static constexpr int TILE_B = 128 * kD * 2;        // one 128 x D tile of 16-bit values
   static constexpr int BIAS_B = 128 * 128 * 2;       // one 128 x 128 bias tile
@@ -92,14 +93,13 @@ __device__ __forceinline__ void put(float (&a)[N], int idx, float v) {
   for (int i = 0; i < N; ++i) a[i] = (idx == i) ? v : a[i];
 }
 
-// kRows: rows per group, FwdCfg::G or 2
-template <int kD, bool kBf16, int kRows>
+template <int kD, bool kBf16>
 __global__ void __launch_bounds__(384, 1)
 fta_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmBias,
                const FwdParams p) {
   using C = FwdCfg<kD>;
-  constexpr int G = C::G;
+  constexpr int G = C::G, kRows = G;
   extern __shared__ uint8_t smem_raw[];
   // 1 KB alignment by an offset from the shared array itself, so that the compiler keeps the
   // shared address space (ld.shared / st.shared instead of generic accesses)
@@ -368,13 +368,10 @@ fta_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         const float alpha = need ? fast_exp2((m_old - m_safe) * kLog2e) : 1.0f;
         if (kb > 0 && __any_sync(0xffffffffu, need)) {
           // The rescale reads and writes the O accumulator of this row, so the row's previous PV MMA
-          // must be done. With two or more rows per warpgroup that was waited for a tile ago; with a
-          // single row the previous tile WAS this row.
-          if constexpr (kRows == 2) {
-            ok = mbar_wait_warp(bar(C::B_PVDONE + wg), (n - 1) & 1, w, 13);
-            if (!ok) break;
-            tc_fence_after_sync();
-          }
+          // (of the warpgroup's previous tile) must be done.
+          ok = mbar_wait_warp(bar(C::B_PVDONE + wg), (n - 1) & 1, w, 13);
+          if (!ok) break;
+          tc_fence_after_sync();
 #pragma unroll
           for (int c = 0; c < kD / 32; ++c) {
             uint32_t orr[32];
@@ -524,12 +521,12 @@ fta_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   if (warp == 0) tmem_dealloc(tbase, 512);
 }
 
-template <int kD, bool kBf16, int kRows>
+template <int kD, bool kBf16>
 int launch_fwd_t(const FwdArgs& a, cudaStream_t stream) {
   using C = FwdCfg<kD>;
-  static_assert(kRows <= C::G && kRows % 2 == 0);
+  constexpr int kRows = C::G;
   static PerDeviceOnce smem_attr;
-  auto kern = fta_fwd_kernel<kD, kBf16, kRows>;
+  auto kern = fta_fwd_kernel<kD, kBf16>;
   if (cudaError_t e = ensure_dynamic_smem(smem_attr, kern, C::SMEM_BYTES)) return static_cast<int>(e);
   FwdParams p;
   p.o = a.o;
@@ -554,16 +551,36 @@ int launch_fwd_t(const FwdArgs& a, cudaStream_t stream) {
 
 }  // namespace
 
+namespace {
+// Key blocks of 64, and whether every pair of rows of a query block has a CTA in one wave of the device
+int key_blocks(int L2) { return (L2 + 63) / 64; }
+bool one_wave(int B, int H, int L1, int L2) {
+  return static_cast<long long>((L2 + 127) / 128) * B * H * ((L1 + 1) / 2) <= num_sms();
+}
+
+// Which kernel: four rows in tiles of 64 keys (fwd_quad_sm100.cu) or the one above, two rows in tiles of 128.
+//  - An odd number of 64-key blocks is half a tile of padding per row for the latter, at D = 32 one that always costs more
+//    (L2 320: 273 us against 328, L2 448: 351 against 407; B2 H8, B1 H8). At D = 64 it pays up to seven blocks (L2 64: 27.5
+//    against 33.8, 320: 384 against 415, 448: 482 against 490): there P replaces S in TMEM, which leaves
+//    the chain of a tile longer, and with an even number the four rows lose (L512: 316 against 291).
+//  - An even number at D = 32: four rows (L256 250 against 265, L768 692 against 720), except where all CTAs of two
+//    rows fit in one wave: with two of its four warpgroups at work nothing covers the hand-over of
+//    its shorter tiles (B1 H8 L1 8 L2 512: 19.5 against 18.5).
+bool use_quad(const int B, const int H, const int L1, const int L2, const int D) {
+  const int n = key_blocks(L2);
+  if (n & 1) return D == 32 || n <= 7;
+  return D == 32 && !one_wave(B, H, L1, L2);
+}
+}  // namespace
+
+int fwd_key_block(int B, int H, int L1, int L2, int D) { return use_quad(B, H, L1, L2, D) ? 64 : 128; }
+
 int launch_fwd(const FwdArgs& a, cudaStream_t stream) {
-  // A problem that leaves SMs idle is bound by the chain of one CTA: groups of two rows (one per softmax
-  // warpgroup) halve it, as long as they all fit in one wave (B1 H4 L64 D32: 14.3 -> 12.3 us a call).
-  // The rows are a template argument: as a run-time value they cost the long problems 4 %.
-  if (a.D == 32) {
-    const long long ctas = static_cast<long long>((a.L2 + 127) / 128) * a.B * a.H * ((a.L1 + 1) / 2);
-    if (ctas <= num_sms()) return a.bf16 ? launch_fwd_t<32, true, 2>(a, stream) : launch_fwd_t<32, false, 2>(a, stream);
-    return a.bf16 ? launch_fwd_t<32, true, 4>(a, stream) : launch_fwd_t<32, false, 4>(a, stream);
-  }
-  return a.bf16 ? launch_fwd_t<64, true, 2>(a, stream) : launch_fwd_t<64, false, 2>(a, stream);
+  // A problem that leaves SMs idle is bound by the chain of one CTA: groups of two rows halve it, as long as they all fit in
+  // one wave. The rows are a template argument: as a run-time value they cost the long problems 4 %.
+  if (use_quad(a.B, a.H, a.L1, a.L2, a.D)) return launch_fwd_quad(a, one_wave(a.B, a.H, a.L1, a.L2), stream);
+  if (a.D == 32) return a.bf16 ? launch_fwd_t<32, true>(a, stream) : launch_fwd_t<32, false>(a, stream);
+  return a.bf16 ? launch_fwd_t<64, true>(a, stream) : launch_fwd_t<64, false>(a, stream);
 }
 
 }  // namespace fta
