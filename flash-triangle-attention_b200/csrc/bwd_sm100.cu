@@ -7,8 +7,8 @@
 // rows in shared memory and dK/dV of the G rows in TMEM, and walks the query blocks `jb`
 // (outer) and the G rows (inner). Per 128 x 128 tile:
 //
-//   S^T  = K Q^T, dP^T = V dO^T                       (tcgen05, operands in smem)
-//   P^T  = exp2((S^T*scale + bias^T - max)*log2e - log2 sum),  dS^T = P^T * (dP^T - delta)   (CUDA cores)
+//   S^T  = K Q^T + c / (scale log2e), dP^T = V dO^T - delta     (tcgen05, operands in smem; c = -(max log2e + log2 sum))
+//   P^T  = exp2(S^T*scale*log2e + bias^T*log2e),  dS^T = P^T * dP^T                          (CUDA cores)
 //   dV  += P^T dO, dK += dS^T Q                        (A operand read from TMEM)
 //   dQ   = dS K                                        (dS staged in smem, M-major)
 //
@@ -35,16 +35,25 @@
 // gets out 32 bytes per cycle of stores and 25 of float32 reductions (30 and 24 with all SMs at it): at D = 32 a tile's
 // 16 KB of dQ and third of 64 KB of dBias need 1 560 cycles, at D = 64 32 KB and 64 KB need 4 100.
 //
-// Measured (main kernel, B1 H4 L1 96 L2 768 D32 bf16): 256 -> 197 us against four quarter-tile warpgroups moving in
-// step through two phases per tile, each phase with its own hand-over. A tile takes about 3 770 cycles, of which a
-// half's pass is 1 500 (512 are its exponentials; two warps per scheduler do not hide the latencies of the
-// chain), hand-over to hand-over 700, and a third of a flush 500. At D = 64 it takes 7 200 (L2 512) to 10 800 (L2 2048, where
-// the planes pass the L2 cache).
+// Measured (whole backward pass, us, before -> with the statistics in the accumulators, the bias loaded a chunk ahead and
+// more registers for the service warps): B1 H4 bf16 L768 1 708 -> 1 641, L512 574 -> 546 (fp16 558 -> 533), B4 H8 L256 fp16 671 ->
+// 662, B2 H8 L160 204 -> 200; D 64: L512 1 019 -> 1 000, B4 H8 L256 1 330 -> 1 321.
+// What bounds it (clock stamps of one CTA, L768 D32, 3 700 cycles a tile): both halves are in their pass together for
+// 2 600 cycles, then wait for the issuer, 600 cycles a half for dV, dK and the next S^T, dP^T, of which 430 are the MMAs
+// themselves (probe: an MMA with M = 128, K = 16 and A in shared memory takes 48 cycles up to N = 64 and 65 at N = 128;
+// with A in TMEM 29 at N = 32). The pass alone takes 1 400 (two warps per scheduler) and 1 900 to 2 000 while the tensor
+// core reads its operands from shared memory, which delays the pass's own accesses there; MMAs with A in TMEM do not. The
+// rest is instruction fetch: all roles together run through more code than the SM's instruction cache holds (6 % of the
+// requests miss, 70 % of the peak rate of the next level), so every role's code counts: a second copy of the poll
+// in each wait made the whole pass 15 % slower.
 // Tried: the four quarters with a hand-over each (768 threads, 96 registers): the issuer, at a good 1 000 cycles per
-// turn, became the bound (3.18 ms at L768 against 2.71); 16 queries per TMEM load instead of 8: equal.
+// turn, became the bound (3.18 ms at L768 against 2.71); 16 queries per TMEM load instead of 8: equal; all of a row's bias
+// loaded before the pass (1 724 us against 1 664 for the pass at L768), the issuer's MMAs in loops instead of unrolled
+// (2 001), its other barriers polled together ahead of the hand-over (1 781), records for 32 queries at a time (2 240),
+// 200 registers for the compute warps and 56 for the others (1 891).
 //
 //   warp 0      : tcgen05 issuer (lowest warp id: the scheduler prefers older warps)
-//   warp 1      : TMA producer        warp 2 : idle        warp 3 : dBias boxes (TMA reductions)
+//   warp 1      : TMA producer        warp 2 : statistics records        warp 3 : dBias boxes (TMA reductions)
 //   warps 4-7   : drain warpgroup (dQ tiles, finished dK / dV rows)
 //   warps 8-15  : two compute warpgroups, one 64-query half of the tile each
 // Producer and issuer loops run warp-uniformly; one elected lane issues the TMA / MMA.
@@ -56,8 +65,9 @@ namespace {
 
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kBwdThreads = 512;
-// registers per thread after setmaxnreg: 2 * 184 + 72 + 72 = 4 * 128, the block's allotment at launch
-constexpr int kRegsCompute = 184, kRegsDrain = 72, kRegsService = 72;
+// registers per thread after setmaxnreg: 2 * 176 + 72 + 88 = 4 * 128, the block's allotment at launch. The service warps
+// (issuer) spill with less than 88.
+constexpr int kRegsCompute = 176, kRegsDrain = 72, kRegsService = 88;
 
 template <int kD>
 struct BwdCfg {
@@ -68,7 +78,7 @@ struct BwdCfg {
   static constexpr bool KV_AHEAD = G >= 3;
   static constexpr int DQS_B = 128 * 16 * 4;  // dQ staging tile: 128 queries x 16 columns, float32
   static constexpr int TILE_B = 128 * kD * 2;
-  static constexpr int STAGE_B = 2 * TILE_B + 2048;  // Q, dO, -max[128], -log2sum[128], delta[128], c[128]
+  static constexpr int STAGE_B = 2 * TILE_B + 2048;  // Q, dO, a 16-byte record of statistics per query
   static constexpr int BIAS_B = 128 * 128 * 2;
   static constexpr int DS_B = 128 * 128 * 2;
   static constexpr int OFF_KV = 0;
@@ -77,8 +87,9 @@ struct BwdCfg {
   static constexpr int OFF_DS = OFF_BIAS + 2 * BIAS_B;
   static constexpr int OFF_DQS = OFF_DS + DS_B;
   static constexpr int OFF_BOX = OFF_DQS + DQS_B;
-  static constexpr int OFF_ZERO = OFF_BOX + NX * 16384;  // 256 zero bytes
-  static constexpr int OFF_BAR = OFF_ZERO + 256;
+  static constexpr int OFF_ONES = OFF_BOX + NX * 16384;  // A operands that pick c / -delta from the records: 2 x 128 rows x 8
+  static constexpr int OFF_ZERO = OFF_ONES + 4096;       // 64 x 8 zeros: the upper half of a record's K = 16
+  static constexpr int OFF_BAR = OFF_ZERO + 1024;
   static constexpr int B_KVFULL = 0;                  // per row of the group
   static constexpr int B_KVFREE = B_KVFULL + G;
   static constexpr int B_QDOFULL = B_KVFREE + G;      // 2 * ring slot + query half
@@ -117,11 +128,16 @@ struct BwdParams {
   long long stat_stride;  // elements between the statistics planes
 };
 
-__device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
-      : "memory");
+// Two numbers as three bfloat16 each (24 bits and more), as the six leading elements of a query's record
+__device__ __forceinline__ uint4 stat_record(float c, float d, uint32_t flags) {
+  const uint32_t h = pack_bf16x2(c, d);
+  c -= __uint_as_float(h << 16);
+  d -= __uint_as_float(h & 0xFFFF0000u);
+  const uint32_t m = pack_bf16x2(c, d);
+  c -= __uint_as_float(m << 16);
+  d -= __uint_as_float(m & 0xFFFF0000u);
+  const uint32_t l = pack_bf16x2(c, d);
+  return make_uint4(__byte_perm(h, m, 0x5410), __byte_perm(l, h, 0x7610), __byte_perm(m, l, 0x7632), flags);
 }
 
 template <int kD, bool kBf16>
@@ -143,6 +159,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   uint8_t* sDS = smem + C::OFF_DS;      // [query half][key row][64 queries], 128B swizzle
   uint8_t* sDQ = smem + C::OFF_DQS;     // float32 dQ tile on its way to the TMA reduction
   uint8_t* sBox = smem + C::OFF_BOX;
+  uint8_t* sOnes = smem + C::OFF_ONES;
   uint8_t* sZero = smem + C::OFF_ZERO;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NBAR);
@@ -174,7 +191,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       mbar_init(bar(C::B_ACCFREE + i), 4);
     }
     for (int i = 0; i < 2 * C::NQ; ++i) {
-      mbar_init(bar(C::B_QDOFULL + i), 1);
+      mbar_init(bar(C::B_QDOFULL + i), 2);  // the producer's expected bytes, the record warp
       mbar_init(bar(C::B_QDOEMPTY + i), 1);
     }
     for (int i = 0; i < 4; ++i) {
@@ -191,7 +208,12 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     }
     mbar_fence_init();
   }
-  if (threadIdx.x < 64) reinterpret_cast<uint32_t*>(sZero)[threadIdx.x] = 0u;
+  if (threadIdx.x < 256) {
+    reinterpret_cast<uint4*>(sOnes)[threadIdx.x] = threadIdx.x < 128 ? make_uint4(0x3F803F80u, 0x00003F80u, 0u, 0u)   // 1 1 1 0 0 0 0 0
+                                                                     : make_uint4(0u, 0xBF800000u, 0xBF80BF80u, 0u);  // 0 0 0 -1 -1 -1 0 0
+    if (threadIdx.x < 64) reinterpret_cast<uint4*>(sZero)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
+    fence_proxy_async_smem();
+  }
   if (warp == 0) {
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
@@ -253,15 +275,9 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 const uint32_t st = smem_u32(sQDO + s * C::STAGE_B);
                 const uint32_t full = bar(C::B_QDOFULL + 2 * s + hf);
                 const int q0 = jb * 128 + hf * 64;
-                mbar_expect_tx(full, C::TILE_B + 1024);
+                mbar_expect_tx(full, C::TILE_B);
                 tma_load_5d_hint(st + hf * C::HALF_B, &tmQ, full, 0, q0, i0 + g, h, b, pol_stream);
                 tma_load_5d_hint(st + C::TILE_B + hf * C::HALF_B, &tmDO, full, 0, q0, i0 + g, h, b, pol_stream);
-                const long long roff = (static_cast<long long>(bh) * p.L1 + i0 + g) * p.stat_pitch + q0;
-                const uint32_t sst = st + 2 * C::TILE_B + hf * 256;
-                bulk_load_1d(sst, p.lse + roff, 256, full);
-                bulk_load_1d(sst + 512, p.lse + p.stat_stride + roff, 256, full);
-                bulk_load_1d(sst + 1024, p.delta + roff, 256, full);
-                bulk_load_1d(sst + 1536, p.lse + 2 * p.stat_stride + roff, 256, full);
               }
               __syncwarp();
               if (g == 0) {  // after the Q/dO loads: the half stages come free later than the ring slot
@@ -297,6 +313,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       constexpr int fmt = kBf16 ? 1 : 0;
       constexpr uint32_t idesc_acc = umma_idesc_f16(fmt, 128, kD, 0, 1);  // dV, dK (A in TMEM, B M-major)
       constexpr uint32_t idesc_x = umma_idesc_f16(fmt, 128, 64, 0, 0);    // S^T, dP^T: 64 queries
+      constexpr uint32_t idesc_st = umma_idesc_f16(1, 128, 64, 0, 0);     // the records' part of S^T, dP^T: bfloat16
       constexpr uint32_t idesc_dq = umma_idesc_f16(fmt, 128, kD, 1, 1);   // dQ (A, B M-major)
       // Descriptors as 32-bit low words (address and leading-dimension offset); the high word is a constant.
       constexpr uint32_t HI = (C::SBO >> 4) | (1u << 14) | (static_cast<uint32_t>(C::SWZ) << 29);
@@ -305,26 +322,34 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       constexpr uint32_t KSTEP = (2 * C::SBO) >> 4;                // 16 rows further (M-major operand)
       const uint32_t lo_kv = smem_u32(sKV) >> 4, lo_qdo = smem_u32(sQDO) >> 4;  // shared addresses are below 2^18
       constexpr uint32_t KV_STEP = 2 * C::TILE_B >> 4, SLOT_STEP = C::STAGE_B >> 4, TILE_STEP = C::TILE_B >> 4,
-                         HALF_STEP = C::HALF_B >> 4;
+                         HALF_STEP = C::HALF_B >> 4, REC_OFF = 2 * C::TILE_B >> 4, REC_HALF = 1024 >> 4;
       bool ok = true, fresh = true;
       int n = 0, jb = 0, g = 0, Gc = min(G, row_end - row_begin), slot = 0, tt = 0;
       uint32_t ring_par = 0;
-      // S^T = K Q^T, dP^T = V dO^T of half hf, by the elected lane; kv, q: low words of K and of the half's Q
-      auto issue_x = [&](int hf, uint32_t kv, uint32_t q) {
+      // The records: rows of 8 elements without a swizzle, 128 bytes per 8 rows; the upper half of K = 16 is zeros on their
+      // side (and whatever finite numbers follow on the other). LBO = distance to it.
+      constexpr uint32_t HI_ST = (128u >> 4) | (1u << 14);
+      auto mk_st = [](uint32_t lo) { return (static_cast<uint64_t>(HI_ST) << 32) | lo; };
+      const uint32_t lo_ones = (smem_u32(sOnes) >> 4) | (128u >> 4) << 16, lo_zero = smem_u32(sZero) >> 4;
+      // S^T = K Q^T + c / (scale log2 e), dP^T = V dO^T - delta of half hf, by the elected lane; kv, q, st: low words of K, of
+      // the half's Q and of its records
+      auto issue_x = [&](int hf, uint32_t kv, uint32_t q, uint32_t st) {
+        const uint64_t rec = mk_st(st | (lo_zero - st) << 16);
+        umma_ss(tbase + C::TM_ST + hf * 64, mk_st(lo_ones), rec, idesc_st, 0);
 #pragma unroll
         for (int ks = 0; ks < kD / 16; ++ks)
-          umma_ss(tbase + C::TM_ST + hf * 64, mk(kv | LK) + ks * 2, mk(q | LK) + ks * 2, idesc_x, ks > 0);
+          umma_ss(tbase + C::TM_ST + hf * 64, mk(kv | LK) + ks * 2, mk(q | LK) + ks * 2, idesc_x, 1);
+        umma_ss(tbase + C::TM_DP + hf * 64, mk_st(lo_ones + (2048 >> 4)), rec, idesc_st, 0);
 #pragma unroll
         for (int ks = 0; ks < kD / 16; ++ks)
-          umma_ss(tbase + C::TM_DP + hf * 64, mk((kv + TILE_STEP) | LK) + ks * 2, mk((q + TILE_STEP) | LK) + ks * 2, idesc_x,
-                  ks > 0);
+          umma_ss(tbase + C::TM_DP + hf * 64, mk((kv + TILE_STEP) | LK) + ks * 2, mk((q + TILE_STEP) | LK) + ks * 2, idesc_x, 1);
         umma_commit(bar(C::B_XFULL + hf));
       };
       auto start_half1 = [&]() -> bool {
         ok = mbar_wait_warp(bar(C::B_QDOFULL + 2 * slot + 1), ring_par, w, 0x35);
         if (!ok) return false;
         tc_fence_after_sync();
-        if (elect_one()) issue_x(1, lo_kv + g * KV_STEP, lo_qdo + slot * SLOT_STEP + HALF_STEP);
+        if (elect_one()) issue_x(1, lo_kv + g * KV_STEP, lo_qdo + slot * SLOT_STEP + HALF_STEP, lo_qdo + slot * SLOT_STEP + REC_OFF + REC_HALF);
         __syncwarp();
         return true;
       };
@@ -334,7 +359,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                mbar_wait_warp(bar(C::B_QDOFULL + 2 * slot), ring_par, w, 0x30);
           if (!ok) break;
           tc_fence_after_sync();
-          if (elect_one()) issue_x(0, lo_kv + g * KV_STEP, lo_qdo + slot * SLOT_STEP);
+          if (elect_one()) issue_x(0, lo_kv + g * KV_STEP, lo_qdo + slot * SLOT_STEP, lo_qdo + slot * SLOT_STEP + REC_OFF);
           __syncwarp();
           if (!C::KV_AHEAD && !start_half1()) break;
         }
@@ -360,8 +385,9 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         for (int hf = 0; hf < 2; ++hf) {
           const uint32_t qv = lo_qdo + slot * SLOT_STEP + hf * HALF_STEP;
           const uint32_t kvn = lo_kv + g1 * KV_STEP, qn = lo_qdo + slot1 * SLOT_STEP + hf * HALF_STEP;
+          const uint32_t stn = lo_qdo + slot1 * SLOT_STEP + REC_OFF + hf * REC_HALF;
           const uint32_t first = (hf || jb > 0) ? 1u : 0u;  // 0: the accumulators start at zero
-          asm volatile("" ::"r"(qv), "r"(kvn), "r"(qn), "r"(first));
+          asm volatile("" ::"r"(qv), "r"(kvn), "r"(qn), "r"(stn), "r"(first));
           if (cont) {
             ok = mbar_wait_warp(bar(C::B_QDOFULL + 2 * slot1 + hf), ring_par1, w, 0x31);
             if (ok && hf == 0 && jb1 == 0) ok = mbar_wait_warp(bar(C::B_KVFULL + g1), n1 & 1, w, 0x36);
@@ -379,7 +405,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
               umma_ts(acc, tbase + C::TM_DP + hf * 64 + ks * 8, mk(qv | LM) + ks * KSTEP, idesc_acc, ks > 0 ? 1u : first);
-            if (cont) issue_x(hf, kvn, qn);
+            if (cont) issue_x(hf, kvn, qn, stn);
             umma_commit(bar(C::B_QDOEMPTY + 2 * slot + hf));
             if (hf == 1 && last) umma_commit(bar(C::B_ACCFULL + g));
           }
@@ -410,6 +436,68 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         slot = slot1;
         ring_par = ring_par1;
         ++tt;
+      }
+    } else if (warp == 2) {
+      // ---------------------------------------------------------------- record warp
+      // c / (scale log2 e) and delta of a query as three bfloat16 each, in 16 bytes: one K = 16 step of the tensor core with
+      // rows of ones adds the first to all of the query's S^T, one with rows of minus ones takes the second from all of its
+      // dP^T. As operands of the pass they would be broadcast loads, and every 16 bytes a thread loads from shared memory
+      // take its port for four cycles per warp, broadcast or not: 1 024 of a tile's 3 800.
+      // A query whose numbers do not go into a record (|c| > 256, where three rounded additions would cost P more than
+      // they do here; infinite or NaN) is flagged and left out; the compute warps then see to it themselves.
+      const float inv_k1 = 1.0f / (p.scale * kLog2e);
+      const float* cp = p.lse + 2 * p.stat_stride;
+      float2 cn[2], dn[2];
+      auto fetch = [&](int i, int jb) {
+        const long long off = (static_cast<long long>(bh) * p.L1 + i) * p.stat_pitch + jb * 128 + 2 * lane;
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          cn[hf] = __ldg(reinterpret_cast<const float2*>(cp + off + hf * 64));
+          dn[hf] = __ldg(reinterpret_cast<const float2*>(p.delta + off + hf * 64));
+        }
+      };
+      bool ok = true;
+      int s = 0;
+      uint32_t ring_par = 1;
+      fetch(row_begin, 0);
+      for (int n = 0; n < ngroups && ok; ++n) {
+        const int i0 = row_begin + n * G;
+        const int Gc = min(G, row_end - i0);
+        for (int jb = 0; jb < nq && ok; ++jb) {
+          for (int g = 0; g < Gc; ++g) {
+            const float2 cv[2] = {cn[0], cn[1]}, dv[2] = {dn[0], dn[1]};
+            const bool wrap_g = g + 1 == Gc, wrap_jb = wrap_g && jb + 1 == nq;
+            const int i1 = wrap_jb ? i0 + G : wrap_g ? i0 : i0 + g + 1;
+            if (i1 < row_end) fetch(i1, wrap_jb ? 0 : wrap_g ? jb + 1 : jb);
+#pragma unroll 1
+            for (int hf = 0; hf < 2; ++hf) {
+              const float2 c = hf ? cv[1] : cv[0], d = hf ? dv[1] : dv[0];
+              // an empty row (c = -inf) needs P = 0 only
+              float cx = c.x < -1.0e30f ? -1.0e30f : c.x, cy = c.y < -1.0e30f ? -1.0e30f : c.y;
+              const bool bigx = !(fabsf(cx) <= 256.f || cx == -1.0e30f), bigy = !(fabsf(cy) <= 256.f || cy == -1.0e30f);
+              cx *= inv_k1;
+              cy *= inv_k1;
+              const bool fx = bigx || !(fabsf(cx) < 1.0e37f) || !(fabsf(d.x) < 1.0e37f);
+              const bool fy = bigy || !(fabsf(cy) < 1.0e37f) || !(fabsf(d.y) < 1.0e37f);
+              const uint32_t any = __any_sync(0xffffffffu, fx || fy) && lane == 0 ? 0x3F800000u : 0u;
+              const uint4 rx = stat_record(fx ? 0.f : cx, fx ? 0.f : d.x, (fx ? 0x3F80u : 0u) | any);
+              const uint4 ry = stat_record(fy ? 0.f : cy, fy ? 0.f : d.y, fy ? 0x3F80u : 0u);
+              ok = mbar_wait_warp(bar(C::B_QDOEMPTY + 2 * s + hf), ring_par, w, 0x24);
+              if (!ok) break;
+              const uint32_t dst = smem_u32(sQDO + s * C::STAGE_B) + 2 * C::TILE_B + hf * 1024 + lane * 32;
+              st_shared_v4(dst, rx.x, rx.y, rx.z, rx.w);
+              st_shared_v4(dst + 16, ry.x, ry.y, ry.z, ry.w);
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar(C::B_QDOFULL + 2 * s + hf));
+            }
+            if (!ok) break;
+            if (++s == C::NQ) {
+              s = 0;
+              ring_par ^= 1u;
+            }
+          }
+        }
       }
     } else if (warp == 3) {
       // ---------------------------------------------------------------- dBias box warp
@@ -553,7 +641,6 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // this half's 64 fp32 columns of S^T / dP^T; P^T / dS^T overwrite the first 32 of them
     const uint32_t tST = tbase + C::TM_ST + hf * 64 + lane_off;
     const uint32_t tDP = tbase + C::TM_DP + hf * 64 + lane_off;
-    const f32x2 neg1_2 = mk2(-1.f, -1.f);
     const uint32_t my_ds = smem_u32(sDS) + hf * 16384 + key * 128;
     bool ok = true;
     int tt = 0, nb = 0, slot = 0;
@@ -574,51 +661,49 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                mbar_wait_warp(bar(C::B_XFULL + hf), tt & 1, w, 0x42);
           if (!ok) break;
           tc_fence_after_sync();
-          const uint8_t* stats = sQDO + slot * C::STAGE_B + 2 * C::TILE_B + hf * 256;
-          const float4* del4 = reinterpret_cast<const float4*>(stats + 1024);
-          const float4* c4 = reinterpret_cast<const float4*>(stats + 1536);
+          const uint4* recs = reinterpret_cast<const uint4*>(sQDO + slot * C::STAGE_B + 2 * C::TILE_B + hf * 1024);
           const uint8_t* brow = sBias + bs * 16384 + key * 128;
           f32x2 k1_2 = mk2(p.scale * kLog2e, p.scale * kLog2e), log2e2 = mk2(kLog2e, kLog2e);
           if (++slot == C::NQ) {
             slot = 0;
             ring_par ^= 1u;
           }
-          // P^T = exp2((S^T*scale + bias^T - max)*log2e - log2 sum) as y = s*(scale*log2e) + (b*log2e + c).
-          // Every lane looks at two of the half's 64 values of c: NaN = a row that needs the two-part form.
-          {
-            const float2 cq = reinterpret_cast<const float2*>(c4)[lane];
-            if (__any_sync(0xffffffffu, cq.x != cq.x || cq.y != cq.y)) {
-              // Rare (rows masked with a large negative bias): form y in a pass of its own, in place of S^T, and
-              // have the pass below take it as it is.
-              const float2* nm2 = reinterpret_cast<const float2*>(stats);
-              const float2* nl2 = reinterpret_cast<const float2*>(stats + 512);
+          // P^T = exp2((S^T*scale + bias^T - max)*log2e - log2 sum) as y = s*(scale*log2e) + b*log2e, with the statistics in s
+          // already, unless a query of the half is flagged.
+          if (recs[0].w != 0u) {
+            // Rare (rows masked with a large negative bias): form y, and dP - delta of the flagged queries, in a pass of its
+            // own, in place of S^T and dP^T, and have the pass below take them as they are.
+            const long long off = (static_cast<long long>(bh) * p.L1 + row_begin + n * G + g) * p.stat_pitch + jb * 128 + hf * 64;
 #pragma unroll 1
-              for (int ch = 0; ch < 8; ++ch) {
-                uint32_t sv[8];
-                tmem_ld8(tST + ch * 8, sv);
-                const uint4 bv = *reinterpret_cast<const uint4*>(brow + ((ch ^ (key & 7)) << 4));
-                const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-                tmem_ld_wait();
+            for (int ch = 0; ch < 8; ++ch) {
+              uint32_t sv[8], dv[8];
+              tmem_ld8(tST + ch * 8, sv);
+              tmem_ld8(tDP + ch * 8, dv);
+              const uint4 bv = *reinterpret_cast<const uint4*>(brow + ((ch ^ (key & 7)) << 4));
+              const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+              tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  float b0, b1, y0, y1;
-                  unpack2<kBf16>(bw[e], b0, b1);
+              for (int e = 0; e < 8; ++e) {
+                float b0, b1;
+                unpack2<kBf16>(bw[e >> 1], b0, b1);
+                const float bq = (e & 1) ? b1 : b0, sq = __uint_as_float(sv[e]);
+                float y = fmaf(sq, p.scale * kLog2e, bq * kLog2e);
+                if (recs[ch * 8 + e].w & 0xFFFFu) {
                   // x = s*scale + b exactly as the forward pass formed it; (x - max) is then exact
                   // for x near the max whatever its magnitude; y = (x - max)*log2e - log2(sum)
-                  const f32x2 x = fma2(mk2(__uint_as_float(sv[2 * e]), __uint_as_float(sv[2 * e + 1])),
-                                       mk2(p.scale, p.scale), mk2(b0, b1));
-                  un2(fma2(add2(x, nm2[ch * 4 + e]), log2e2, nl2[ch * 4 + e]), y0, y1);
-                  sv[2 * e] = __float_as_uint(y0);
-                  sv[2 * e + 1] = __float_as_uint(y1);
+                  const long long o = off + ch * 8 + e;
+                  y = fmaf(fmaf(sq, p.scale, bq) + __ldg(p.lse + o), kLog2e, __ldg(p.lse + p.stat_stride + o));
+                  dv[e] = __float_as_uint(__uint_as_float(dv[e]) - __ldg(p.delta + o));
                 }
-                tmem_st8(tST + ch * 8, sv);
+                sv[e] = __float_as_uint(y);
               }
-              tmem_st_wait();
-              k1_2 = mk2(1.f, 1.f);
-              log2e2 = mk2(0.f, 0.f);
-              c4 = reinterpret_cast<const float4*>(sZero);
-              brow = sZero;
+              tmem_st8(tST + ch * 8, sv);
+              tmem_st8(tDP + ch * 8, dv);
             }
+            tmem_st_wait();
+            k1_2 = mk2(1.f, 1.f);
+            log2e2 = mk2(0.f, 0.f);
+            brow = sZero;
           }
           // One pass over the 64 queries in chunks of 8: S^T and dP^T of a chunk are loaded while the previous one is
           // worked on. P^T (input dtype) and dS^T = P^T * (dP^T - delta), with P in float32, replace them in
@@ -626,34 +711,34 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           uint32_t dd[32], ds_free = 1;
           {
             uint32_t sv[2][8], dv[2][8], pp[8];
+            uint4 bv[2];
+            auto load_bias = [&](int ch) { return *reinterpret_cast<const uint4*>(brow + ((ch ^ (key & 7)) << 4)); };
             tmem_ld8(tST, sv[0]);
             tmem_ld8(tDP, dv[0]);
+            bv[0] = load_bias(0);
             tmem_ld_wait();
 #pragma unroll
             for (int ch = 0; ch < 8; ++ch) {
               if (ch < 7) {
                 tmem_ld8(tST + (ch + 1) * 8, sv[(ch + 1) & 1]);
                 tmem_ld8(tDP + (ch + 1) * 8, dv[(ch + 1) & 1]);
+                // a chunk ahead like them: nothing moves across the wait below, and a load behind it shows its latency
+                // (the pass alone, two warps per scheduler: 1 700 -> 1 390 cycles; one: 1 310 -> 910)
+                bv[(ch + 1) & 1] = load_bias(ch + 1);
               }
               if (ch == 4 && tt > 0) ds_free = mbar_test_wait(bar(C::B_DQDONE + ((tt - 1) & 1)), ((tt - 1) >> 1) & 1);
-              const uint4 bv = *reinterpret_cast<const uint4*>(brow + ((ch ^ (key & 7)) << 4));
-              const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-              const float4 ca = c4[ch * 2], cb = c4[ch * 2 + 1];
-              const f32x2 c2[4] = {mk2(ca.x, ca.y), mk2(ca.z, ca.w), mk2(cb.x, cb.y), mk2(cb.z, cb.w)};
-              const float4 da = del4[ch * 2], db = del4[ch * 2 + 1];
-              const f32x2 del2[4] = {mk2(da.x, da.y), mk2(da.z, da.w), mk2(db.x, db.y), mk2(db.z, db.w)};
+              const uint32_t bw[4] = {bv[ch & 1].x, bv[ch & 1].y, bv[ch & 1].z, bv[ch & 1].w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 float b0, b1, y0, y1, ds0, ds1;
                 unpack2<kBf16>(bw[e], b0, b1);
                 un2(fma2(mk2(__uint_as_float(sv[ch & 1][2 * e]), __uint_as_float(sv[ch & 1][2 * e + 1])), k1_2,
-                         fma2(mk2(b0, b1), log2e2, c2[e])),
+                         mul2(mk2(b0, b1), log2e2)),
                     y0, y1);
                 const float p0 = fast_exp2(y0), p1 = fast_exp2(y1);
                 pp[(ch & 1) * 4 + e] = pack2<kBf16>(p0, p1);
-                const f32x2 u = fma2(del2[e], neg1_2,
-                                     mk2(__uint_as_float(dv[ch & 1][2 * e]), __uint_as_float(dv[ch & 1][2 * e + 1])));
-                const f32x2 ds = mul2(mk2(p0, p1), u);
+                const f32x2 ds =
+                    mul2(mk2(p0, p1), mk2(__uint_as_float(dv[ch & 1][2 * e]), __uint_as_float(dv[ch & 1][2 * e + 1])));
                 acc[ch * 4 + e] = add2(acc[ch * 4 + e], ds);
                 un2(ds, ds0, ds1);
                 dd[ch * 4 + e] = pack2<kBf16>(ds0, ds1);
@@ -669,7 +754,7 @@ fta_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                     st_shared_v4(my_ds + ((j ^ (key & 7)) << 4), dd[4 * j], dd[4 * j + 1], dd[4 * j + 2], dd[4 * j + 3]);
                 }
               }
-              // the 16 columns of queries 16i .. 16i+15 have been read: their results go to columns 8i .. 8i+7
+              // the 8 columns of this chunk have been read: their results go to columns 4 ch .. 4 ch + 3
               if (ch & 1) {
                 tmem_st8(tST + (ch >> 1) * 8, pp);
                 tmem_st8(tDP + (ch >> 1) * 8, dd + (ch >> 1) * 8);

@@ -18,7 +18,7 @@
 // own instructions: with one for all four rows it was the bound (L768 forward 850 us; two: 692). A warp for each row
 // that also does the row's loads is never waited for, and yet slower (736): the softmax warps are then in step often enough
 // to queue for the exp2 unit. Issuing from the softmax warps themselves: 933.
-// The bias is loaded two vectors ahead of its use (four: 703, none: 720).
+// The bias is loaded two vectors ahead of its use (four: 703).
 //
 // Measured (two warpgroups with tiles of 128 keys -> this kernel, us, D 32 bf16 unless stated): inference B1 H4 L768 722 ->
 // 685, L384 105.6 -> 101.4, B4 H8 L256 263 -> 249, L64 29.5 -> 21.4, B1 H8 L317 fp16 174 -> 139, B1 H16 L1 1024 L2 32 136 -> 72,
