@@ -118,7 +118,7 @@ int forward(const FtaProblem* prob, const FtaTensor5* q, const FtaTensor5* k, co
   if (!status.word) return FTA_ERR_NULL;
   if (!aligned16(lse) || !aligned16(o_resid)) return FTA_ERR_ALIGN;
   fta::FwdArgs a;
-  const uint32_t keys = static_cast<uint32_t>(fta::fwd_key_block(prob->B, prob->H, prob->L1, prob->L2, prob->D));
+  const uint32_t keys = static_cast<uint32_t>(fta::fwd_key_block(prob->L2, prob->D));
   if ((rc = map5(&a.tmQ, prob, q)) || (rc = map5(&a.tmK, prob, k, keys)) || (rc = map5(&a.tmV, prob, v, keys)) ||
       (rc = map_bias(&a.tmBias, prob, bias, 64, 128)))
     return rc;

@@ -89,10 +89,10 @@ struct FwdArgs {
   float sm_scale;
 };
 int launch_fwd(const FwdArgs& a, cudaStream_t stream);
-// launch_fwd's kernel with tiles of 64 keys; `two_rows`: groups of two rows instead of four
-int launch_fwd_quad(const FwdArgs& a, bool two_rows, cudaStream_t stream);
+// launch_fwd's kernel with tiles of 64 keys
+int launch_fwd_quad(const FwdArgs& a, cudaStream_t stream);
 // keys per K / V tile of the kernel that launch_fwd takes for a problem: the box height of FwdArgs::tmK and tmV
-int fwd_key_block(int B, int H, int L1, int L2, int D);
+int fwd_key_block(int L2, int D);
 
 struct BwdArgs {
   CUtensorMap tmQ, tmK, tmV, tmDO, tmBiasT;  // tmBiasT: over the key-major copy of the bias

@@ -77,8 +77,10 @@ struct QuadCfg {
   static constexpr uint32_t TM_O = P_OVER_S ? 256 : 384;     // + D g
   static_assert(TM_O + G * kD <= 512, "TMEM budget");
 };
-constexpr int kQuadThreads = 640;
-// registers per thread after setmaxnreg: 512 * 104 + 128 * 64 = 640 * 96, the block's allotment at launch
+// threads of a block: four service warps, kRows softmax warpgroups
+constexpr int quad_threads(int rows) { return 128 + 128 * rows; }
+// registers per thread after setmaxnreg with four rows: 512 * 104 + 128 * 64 = 640 * 96, the block's allotment at launch;
+// a block of two rows has 168 for every thread
 constexpr int kRegsSoftmax = 104, kRegsService = 64;
 
 struct QuadParams {
@@ -94,9 +96,9 @@ struct QuadParams {
   long long stat_stride;             // elements between the statistics planes
 };
 
-// kRows: rows per group (the warpgroups beyond it are idle)
+// kRows: rows per group == softmax warpgroups
 template <int kD, bool kBf16, int kRows>
-__global__ void __launch_bounds__(kQuadThreads, 1)
+__global__ void __launch_bounds__(quad_threads(kRows), 1)
 fta_fwd_quad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmBias,
                const QuadParams p) {
@@ -162,7 +164,7 @@ fta_fwd_quad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   grid_dependency_wait();
 
   if (warp < 4) {
-    reg_dec<kRegsService>();
+    if constexpr (kRows == 4) reg_dec<kRegsService>();
     if (warp == 1) {
       // ---------------------------------------------------------------- TMA producer
       if (elect_one()) {
@@ -306,9 +308,9 @@ fta_fwd_quad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (++kb == nkb) kb = 0;
       }
     }
-  } else if (warp < 4 + 4 * kRows) {
+  } else {
     // ------------------------------------------------------------------ softmax warpgroups
-    reg_inc<kRegsSoftmax>();
+    if constexpr (kRows == 4) reg_inc<kRegsSoftmax>();
     const int g = (warp >> 2) - 1;           // warpgroup == row of the group
     const int row = (warp & 3) * 32 + lane;  // query row of the tile == TMEM lane
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
@@ -327,9 +329,10 @@ fta_fwd_quad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const uint8_t* brow = sBias + bs * C::BIAS_B + row * 128;
         ok = mbar_finish_wait(b_in, bar(C::B_BIASFULL + bs), bias_par, w, 7);
         if (!ok) break;
+        constexpr int kAhead = kRows == 4 ? 2 : 7;  // vectors of the bias loaded before S; with four rows no register is left for more
         uint4 bv[8];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) bv[c] = *reinterpret_cast<const uint4*>(brow + ((c ^ (row & 7)) << 4));
+        for (int c = 0; c < kAhead; ++c) bv[c] = *reinterpret_cast<const uint4*>(brow + ((c ^ (row & 7)) << 4));
         ok = mbar_finish_wait(s_in, bar(C::B_SFULL + g), n & 1, w, 6);
         if (!ok) break;
         tc_fence_after_sync();
@@ -350,7 +353,7 @@ fta_fwd_quad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          if (c < 6) bv[c + 2] = *reinterpret_cast<const uint4*>(brow + (((c + 2) ^ (row & 7)) << 4));
+          if (c < 8 - kAhead) bv[c + kAhead] = *reinterpret_cast<const uint4*>(brow + (((c + kAhead) ^ (row & 7)) << 4));
           const uint32_t bw[4] = {bv[c].x, bv[c].y, bv[c].z, bv[c].w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
@@ -545,8 +548,7 @@ int launch_quad_t(const FwdArgs& a, cudaStream_t stream) {
   p.H = a.H;
   p.L1 = a.L1;
   p.L2 = a.L2;
-  // whole 32-byte sectors per store: 16 bytes at a time, 64 or 128 apart from lane to lane, an SM's way out carries each
-  // sector twice
+  // whole 32-byte sectors per store: 16 bytes at a time, 64 or 128 apart from lane to lane, each sector leaves the SM twice
   p.wide = (reinterpret_cast<uintptr_t>(a.o) | reinterpret_cast<uintptr_t>(a.o_resid)) % 32 == 0 && a.so[0] % 16 == 0 &&
            a.so[1] % 16 == 0 && a.so[2] % 16 == 0 && a.so[3] % 16 == 0;
   p.so_b = a.so[0];
@@ -559,12 +561,15 @@ int launch_quad_t(const FwdArgs& a, cudaStream_t stream) {
   const long long per = static_cast<long long>((a.L2 + 127) / 128) * a.B * a.H;
   const int grid_y = fwd_grid_rows((a.L1 + kRows - 1) / kRows, per, num_sms());
   dim3 grid((a.L2 + 127) / 128, grid_y, a.B * a.H);
-  return static_cast<int>(launch_overlapped(kern, grid, kQuadThreads, C::SMEM_BYTES, stream, a.tmQ, a.tmK, a.tmV, a.tmBias, p));
+  return static_cast<int>(launch_overlapped(kern, grid, quad_threads(kRows), C::SMEM_BYTES, stream, a.tmQ, a.tmK, a.tmV, a.tmBias, p));
 }
 
 }  // namespace
 
-int launch_fwd_quad(const FwdArgs& a, bool two_rows, cudaStream_t stream) {
+int launch_fwd_quad(const FwdArgs& a, cudaStream_t stream) {
+  // A problem that leaves SMs idle is bound by the chain of one CTA: groups of two rows halve it, as long as they all fit in
+  // one wave. The rows are a template argument: as a run-time value they cost the long problems 4 %.
+  const bool two_rows = static_cast<long long>((a.L2 + 127) / 128) * a.B * a.H * ((a.L1 + 1) / 2) <= num_sms();
   auto go = [&](auto d) {
     constexpr int D = decltype(d)::value;
     if (two_rows) return a.bf16 ? launch_quad_t<D, true, 2>(a, stream) : launch_quad_t<D, false, 2>(a, stream);

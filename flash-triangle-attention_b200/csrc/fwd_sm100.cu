@@ -1,6 +1,6 @@
 // Forward triangle attention for sm_100a: O = softmax(sm_scale * q k^T + bias) v and the
 // softmax statistics (row max and log2 of the row sum), the work of the reference's `_attn_fwd` (flash_tt_attn.py:128-264).
-// For D = 64 with more than a few key blocks and for small problems; the others go to fwd_quad_sm100.cu (see launch_fwd).
+// For D = 64 with more than a few key blocks; the others go to fwd_quad_sm100.cu (see use_quad).
 //
 // One CTA owns a 128-query block `jb` of one (b,h) and walks a residue class of the groups of G
 // consecutive L1 rows back to back (loads and MMAs of the next group start while the softmax
@@ -41,7 +41,8 @@ constexpr float kLog2e = 1.4426950408889634f;
 template <int kD>
 struct FwdCfg {
   static constexpr int G = 2;                        // rows per group, one per softmax warpgroup
-  static constexpr int NSTAGE = (kD == 32) ? 6 : 4;  // K/V ring depth
+  static_assert(kD == 64);                           // D = 32 goes to the kernel with four rows
+  static constexpr int NSTAGE = 4;                   // K/V ring depth
   static constexpr int TILE_B = 128 * kD * 2;        // one 128 x D tile of 16-bit values
   static constexpr int BIAS_B = 128 * 128 * 2;       // one 128 x 128 bias tile
   static constexpr int OFF_Q = 0;
@@ -61,7 +62,7 @@ struct FwdCfg {
   static constexpr int B_PVDONE = B_PFULL + 2;
   static constexpr int NBAR = B_PVDONE + 2;
   static constexpr int SMEM_BYTES = OFF_BAR + NBAR * 8 + 16 + 1024;  // + tmem slot/abort + align slack
-  static constexpr uint64_t SWZ = (kD == 32) ? kSwz64 : kSwz128;
+  static constexpr uint64_t SWZ = kSwz128;
   static constexpr uint32_t SBO = 8 * kD * 2;  // bytes between 8-row groups of a tile
   static constexpr uint32_t TMEM_P = 256;      // first P column
   static constexpr uint32_t TMEM_O = 384;      // first O column
@@ -552,34 +553,24 @@ int launch_fwd_t(const FwdArgs& a, cudaStream_t stream) {
 }  // namespace
 
 namespace {
-// Key blocks of 64, and whether every pair of rows of a query block has a CTA in one wave of the device
-int key_blocks(int L2) { return (L2 + 63) / 64; }
-bool one_wave(int B, int H, int L1, int L2) {
-  return static_cast<long long>((L2 + 127) / 128) * B * H * ((L1 + 1) / 2) <= num_sms();
-}
-
-// Which kernel: four rows in tiles of 64 keys (fwd_quad_sm100.cu) or the one above, two rows in tiles of 128.
-//  - An odd number of 64-key blocks is half a tile of padding per row for the latter, at D = 32 one that always costs more
-//    (L2 320: 273 us against 328, L2 448: 351 against 407; B2 H8, B1 H8). At D = 64 it pays up to seven blocks (L2 64: 27.5
-//    against 33.8, 320: 384 against 415, 448: 482 against 490): there P replaces S in TMEM, which leaves
-//    the chain of a tile longer, and with an even number the four rows lose (L512: 316 against 291).
-//  - An even number at D = 32: four rows (L256 250 against 265, L768 692 against 720), except where all CTAs of two
-//    rows fit in one wave: with two of its four warpgroups at work nothing covers the hand-over of
-//    its shorter tiles (B1 H8 L1 8 L2 512: 19.5 against 18.5).
-bool use_quad(const int B, const int H, const int L1, const int L2, const int D) {
-  const int n = key_blocks(L2);
-  if (n & 1) return D == 32 || n <= 7;
-  return D == 32 && !one_wave(B, H, L1, L2);
+// Which kernel: four rows in tiles of 64 keys (fwd_quad_sm100.cu) or the one above, two rows in tiles of 128. By L2 and D
+// alone: the kernels round O differently, and a block or a rank's share of the rows gives the bits that
+// the whole gives. Training forward, us, bf16, the one above -> four rows:
+//  - D = 32: always four rows (with tiles of 128 keys, groups of four rows over two warpgroups took 765 at B1 H4 L768, four
+//    warpgroups 699).
+//  - D = 64: there P replaces S in TMEM, which leaves the chain of a tile longer. It pays up to six blocks of 64 keys (B4 H8
+//    L256 500 -> 390, inference 345 -> 329; from eight on inference loses: H4 L512 289 -> 297), with an odd number, which the
+//    one above pads to the next even one, up to eleven (inference H8 L320 216 -> 190).
+bool use_quad(const int L2, const int D) {
+  const int n = (L2 + 63) / 64;
+  return D == 32 || n <= 7 || n == 9 || n == 11;
 }
 }  // namespace
 
-int fwd_key_block(int B, int H, int L1, int L2, int D) { return use_quad(B, H, L1, L2, D) ? 64 : 128; }
+int fwd_key_block(int L2, int D) { return use_quad(L2, D) ? 64 : 128; }
 
 int launch_fwd(const FwdArgs& a, cudaStream_t stream) {
-  // A problem that leaves SMs idle is bound by the chain of one CTA: groups of two rows halve it, as long as they all fit in
-  // one wave. The rows are a template argument: as a run-time value they cost the long problems 4 %.
-  if (use_quad(a.B, a.H, a.L1, a.L2, a.D)) return launch_fwd_quad(a, one_wave(a.B, a.H, a.L1, a.L2), stream);
-  if (a.D == 32) return a.bf16 ? launch_fwd_t<32, true>(a, stream) : launch_fwd_t<32, false>(a, stream);
+  if (use_quad(a.L2, a.D)) return launch_fwd_quad(a, stream);
   return a.bf16 ? launch_fwd_t<64, true>(a, stream) : launch_fwd_t<64, false>(a, stream);
 }
 
