@@ -43,8 +43,8 @@
 // themselves (probe: an MMA with M = 128, K = 16 and A in shared memory takes 48 cycles up to N = 64 and 65 at N = 128;
 // with A in TMEM 29 at N = 32). The pass alone takes 1 400 (two warps per scheduler) and 1 900 to 2 000 while the tensor
 // core reads its operands from shared memory, which delays the pass's own accesses there; MMAs with A in TMEM do not. The
-// rest is instruction fetch: all roles together run through more code than the SM's instruction cache holds (6 % of the
-// requests miss, 70 % of the peak rate of the next level), so every role's code counts: a second copy of the poll
+// rest is instruction fetch: all roles together run through more code than the SM's instruction cache holds (6.6 % of the
+// requests miss, 66 % of the peak rate of the next level), so every role's code counts: a second copy of the poll
 // in each wait made the whole pass 15 % slower.
 // Tried: the four quarters with a hand-over each (768 threads, 96 registers): the issuer, at a good 1 000 cycles per
 // turn, became the bound (3.18 ms at L768 against 2.71); 16 queries per TMEM load instead of 8: equal; all of a row's bias

@@ -560,7 +560,8 @@ namespace {
 //    warpgroups 699).
 //  - D = 64: there P replaces S in TMEM, which leaves the chain of a tile longer. It pays up to six blocks of 64 keys (B4 H8
 //    L256 500 -> 390, inference 345 -> 329; from eight on inference loses: H4 L512 289 -> 297), with an odd number, which the
-//    one above pads to the next even one, up to eleven (inference H8 L320 216 -> 190).
+//    one above pads to the next even one, up to eleven (inference H8 L320 216 -> 189, H8 L576 919 -> 898, H4
+//    L704 800 -> 781; an even one before the limit, H8 L384: 252 and 252, with statistics 338 -> 285).
 bool use_quad(const int L2, const int D) {
   const int n = (L2 + 63) / 64;
   return D == 32 || n <= 7 || n == 9 || n == 11;
