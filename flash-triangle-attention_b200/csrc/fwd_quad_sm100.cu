@@ -79,9 +79,13 @@ struct QuadCfg {
 };
 // threads of a block: four service warps, kRows softmax warpgroups
 constexpr int quad_threads(int rows) { return 128 + 128 * rows; }
-// registers per thread after setmaxnreg with four rows: 512 * 104 + 128 * 64 = 640 * 96, the block's allotment at launch;
-// a block of two rows has 168 for every thread
-constexpr int kRegsSoftmax = 104, kRegsService = 64;
+// Registers per thread after setmaxnreg with four rows: 4 * 104 + 64 = 4 * 112 + 32 = 5 * 96, the block's allotment at launch. At
+// D = 64 the softmax warps spill less with 112 than the service warps lose with 32 (B1 H8 L320 training forward 218 -> 208 us,
+// inference 190 -> 181); at D = 32, where 104 nearly suffice, it costs L768 0.6 %. A block of two rows has 168 for every thread.
+template <int kD>
+constexpr int kRegsSoftmax = kD == 32 ? 104 : 112;
+template <int kD>
+constexpr int kRegsService = kD == 32 ? 64 : 32;
 
 struct QuadParams {
   void* o;
@@ -164,7 +168,7 @@ fta_fwd_quad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   grid_dependency_wait();
 
   if (warp < 4) {
-    if constexpr (kRows == 4) reg_dec<kRegsService>();
+    if constexpr (kRows == 4) reg_dec<kRegsService<kD>>();
     if (warp == 1) {
       // ---------------------------------------------------------------- TMA producer
       if (elect_one()) {
@@ -310,7 +314,7 @@ fta_fwd_quad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
   } else {
     // ------------------------------------------------------------------ softmax warpgroups
-    if constexpr (kRows == 4) reg_inc<kRegsSoftmax>();
+    if constexpr (kRows == 4) reg_inc<kRegsSoftmax<kD>>();
     const int g = (warp >> 2) - 1;           // warpgroup == row of the group
     const int row = (warp & 3) * 32 + lane;  // query row of the tile == TMEM lane
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
