@@ -558,10 +558,10 @@ namespace {
 // the whole gives. Training forward, us, bf16, the one above -> four rows:
 //  - D = 32: always four rows (with tiles of 128 keys, groups of four rows over two warpgroups took 765 at B1 H4 L768, four
 //    warpgroups 699).
-//  - D = 64: there P replaces S in TMEM, which leaves the chain of a tile longer. It pays up to six blocks of 64 keys (B4 H8
-//    L256 500 -> 390, inference 345 -> 329; from eight on inference loses: H4 L512 289 -> 297), with an odd number, which the
-//    one above pads to the next even one, up to eleven (inference H8 L320 216 -> 189, H8 L576 919 -> 898, H4
-//    L704 800 -> 781; an even one before the limit, H8 L384: 252 and 252, with statistics 338 -> 285).
+//  - D = 64: there P replaces S in TMEM, which leaves the chain of a tile longer. Up to six blocks of 64 keys it pays throughout
+//    (B4 H8 L256 500 -> 390, inference 345 -> 329; H8 L384 338 -> 282, 252 -> 242), with an odd number, which the one above pads
+//    to the next even one, up to eleven (H8 L576 1 131 -> 937, 919 -> 857; H4 L704 957 -> 798, 800 -> 757). At eight it depends on
+//    how the groups of rows fill the device (H4 L1 512 365 -> 320, 291 -> 289; H8 L1 256 370 -> 344, 294 -> 305).
 bool use_quad(const int L2, const int D) {
   const int n = (L2 + 63) / 64;
   return D == 32 || n <= 7 || n == 9 || n == 11;
